@@ -1,6 +1,5 @@
 // Host side of the dense projections: TMA descriptors, tile selection, launch
-// of the tcgen05 kernel (gemm_sm100.cuh) for bf16/fp16, and a plain FFMA kernel
-// for fp32 (the fp32 configuration is a parity case, not a throughput target).
+// of the tcgen05 kernel (gemm_sm100.cuh) for bf16/fp16 (fp32: gemm_f32.cu).
 #include "gemm_host.cuh"
 
 #include <mutex>
@@ -369,51 +368,6 @@ int run_gemm_sm100(int dtype, int epi, const GemmPlan& plan, const void* x, int6
   if (dtype == SB200_F16) return dispatch_epi<__half>(epi, ta, tb, g, cv, ra, s);
   set_error("tcgen05 GEMM supports bf16/fp16 only");
   return SB200_ERR_UNSUPPORTED;
-}
-
-// --------------------------------------------------------------- fp32 (FFMA)
-// C[M,N] = A[M,K] * B[N,K]^T (+bias), 64x64 tiles, 4x4 outputs per thread.
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(float* __restrict__ C, int64_t ldc, const float* __restrict__ A, int64_t lda,
-                const float* __restrict__ B, int64_t ldb, const float* __restrict__ bias, int M, int N, int K) {
-  __shared__ float sa[16][64 + 1], sb[16][64 + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-      const int r = i >> 4, kk = i & 15;
-      sa[kk][r] = (m0 + r < M && k0 + kk < K) ? A[(int64_t)(m0 + r) * lda + k0 + kk] : 0.f;
-      sb[kk][r] = (n0 + r < N && k0 + kk < K) ? B[(int64_t)(n0 + r) * ldb + k0 + kk] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) { a[i] = sa[kk][ty * 4 + i]; b[i] = sb[kk][tx * 4 + i]; }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-      if (m < M && n < N) C[(int64_t)m * ldc + n] = acc[i][j] + (bias ? bias[n] : 0.f);
-    }
-}
-
-int run_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, const float* B, int64_t ldb, const float* bias,
-                 int M, int N, int K, cudaStream_t s) {
-  dim3 grid((N + 63) / 64, (M + 63) / 64);
-  gemm_f32_kernel<<<grid, 256, 0, s>>>(C, ldc, A, lda, B, ldb, bias, M, N, K);
-  SB_CHECK_LAUNCH("gemm_f32_kernel");
-  return SB200_OK;
 }
 
 }  // namespace sb200

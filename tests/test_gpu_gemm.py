@@ -93,6 +93,25 @@ def test_linear(dtype, tile_n, T, N, K):
     assert rel_err(outb.float(), ref + b.float().cuda()) <= GEMM_TOL[dtype]
 
 
+# tile edges of the fp32 kernel (32 / 64 rows, 128 columns, 16 k), K cut over 1..8 CTAs, rows that are not 16-byte aligned
+@pytest.mark.parametrize("T,N,K", [(1, 1, 1), (32, 128, 4096), (33, 129, 1023), (31, 5, 64), (64, 640, 68), (65, 257, 2816),
+                                   (288, 1536, 1024), (512, 128, 130)])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_linear_f32_tiles(T, N, K, pad):
+    from sarathi_serve_b200 import dense_ops
+    x = _rand((T, K + pad), torch.float32, T + N + K).cuda()[:, pad:]
+    w = _rand((N, K + pad), torch.float32, 7 * N + K).cuda()[:, pad:]
+    b = _rand((N,), torch.float32, 3).cuda()
+    out = torch.full((T, N + pad), 7.0, device="cuda")
+    dense_ops.linear(x, w, b, out=out[:, pad:])
+    ref = x.double() @ w.double().t() + b.double()
+    # K products and K + 9 sums, each rounded once to fp32: |err| <= (K + 10) * 2^-24 * sum |x||w|; random signs leave
+    # about the square root of that many roundings
+    bound = 4 * (K + 10) ** 0.5 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t() + b.double().abs())
+    assert bool(((out[:, pad:].double() - ref).abs() <= bound).all())
+    assert pad == 0 or bool((out[:, :pad] == 7.0).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("tile_n", [0, 128, 3256, 203128, 2064, 205256, 405128])
 @pytest.mark.parametrize("T,N,K", [(512, 4096, 512), (65, 200, 264), (300, 1000, 1000), (1, 256, 512)])
