@@ -700,7 +700,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -768,7 +768,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0 && leader) {
+    if (leader && ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int used = 0;  // tiles actually computed (selects the TMEM buffer)

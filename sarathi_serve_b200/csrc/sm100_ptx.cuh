@@ -5,8 +5,8 @@
 #pragma once
 
 #include <cuda.h>
-#include <cuda_runtime.h>
-#include <stdint.h>
+
+#include "common.cuh"
 
 namespace sb200 {
 namespace ptx {
@@ -15,13 +15,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// ------------------------------------------- programmatic dependent launch
-// A kernel launched with the programmatic-stream-serialization attribute may start while the kernel
-// before it in the stream is still running: `grid_dependency_wait` blocks until that kernel has
-// completed and its memory is visible (a no-op without the attribute); `grid_launch_dependents` lets the
-// NEXT kernel of the stream be scheduled as soon as every CTA of this one has executed it and an SM is free.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// One lane of a converged warp, chosen by the hardware.  Code guarded by this predicate (not by `lane == 0`) is known
+// to run on a single lane, so the instructions that take their operands from uniform registers -- TMA, tcgen05.mma,
+// tcgen05.commit -- are issued directly; under a plain lane test the compiler has to assume several active lanes and
+// wraps every one of them in a loop over the lanes, which cost the MMA and TMA threads about 550 clocks per k-block.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
+}
 
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
