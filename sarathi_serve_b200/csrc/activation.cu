@@ -31,6 +31,7 @@ template <typename T> __device__ __forceinline__ float gelu_fast_op(float x) {
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 silu_and_mul_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t T_, int64_t d) {
+  grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   if constexpr (VEC) {
@@ -75,6 +76,7 @@ silu_and_mul_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t T_, i
 template <typename T, int OP, bool VEC>
 __global__ void __launch_bounds__(256)
 unary_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t total) {
+  grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -114,9 +116,9 @@ static int launch_silu(void* out, const void* in, int64_t T_, int64_t d, cudaStr
   constexpr int N = Vec16<T>::N;
   const bool vec = (d % N == 0) && aligned16(out) && aligned16(in);
   if (vec)
-    silu_and_mul_kernel<T, true><<<grid_for(T_ * (d / N), 256), 256, 0, s>>>((T*)out, (const T*)in, T_, d);
+    launch_dependent(silu_and_mul_kernel<T, true>, grid_for(T_ * (d / N), 256), 256, 0, s, (T*)out, (const T*)in, T_, d);
   else
-    silu_and_mul_kernel<T, false><<<grid_for(T_ * d, 256), 256, 0, s>>>((T*)out, (const T*)in, T_, d);
+    launch_dependent(silu_and_mul_kernel<T, false>, grid_for(T_ * d, 256), 256, 0, s, (T*)out, (const T*)in, T_, d);
   SB_CHECK_LAUNCH("silu_and_mul_kernel");
   return SB200_OK;
 }
@@ -126,9 +128,9 @@ static int launch_unary(void* out, const void* in, int64_t total, cudaStream_t s
   constexpr int N = Vec16<T>::N;
   const bool vec = aligned16(out) && aligned16(in);
   if (vec)
-    unary_kernel<T, OP, true><<<grid_for(total / N + 1, 256), 256, 0, s>>>((T*)out, (const T*)in, total);
+    launch_dependent(unary_kernel<T, OP, true>, grid_for(total / N + 1, 256), 256, 0, s, (T*)out, (const T*)in, total);
   else
-    unary_kernel<T, OP, false><<<grid_for(total, 256), 256, 0, s>>>((T*)out, (const T*)in, total);
+    launch_dependent(unary_kernel<T, OP, false>, grid_for(total, 256), 256, 0, s, (T*)out, (const T*)in, total);
   SB_CHECK_LAUNCH("activation unary_kernel");
   return SB200_OK;
 }

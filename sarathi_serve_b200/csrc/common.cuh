@@ -66,6 +66,39 @@ template <> __device__ __forceinline__ float rt<float>(float v) { return v; }
 
 __host__ __device__ inline size_t dtype_size(int dt) { return dt == SB200_F32 ? 4 : 2; }
 
+// ------------------------------------------- programmatic dependent launch
+// The kernels of this library are launched with the programmatic-stream-serialization attribute: a kernel may start
+// while the one before it in the stream is still running.  `grid_dependency_wait` blocks until that kernel has
+// completed and its memory is visible (a no-op without the attribute); every kernel executes it before its first
+// access to global memory, and completes only after that, so a wait covers all earlier work of the stream.
+// `grid_launch_dependents` lets the NEXT kernel of the stream be scheduled as soon as every CTA of this one has
+// executed it and an SM has room: what overlaps is launch latency and prologues.  A kernel that owns TMEM executes it
+// after its allocation, so that no CTA of a later kernel can hold the TMEM an earlier one still needs.
+// (2048 x 28672 x 4096 back to back: 318 -> 312 us; 300 x 4096 x 4096: 25.6 -> 23.6 us.)
+namespace ptx {
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+}  // namespace ptx
+// Both, for kernels whose prologue is not worth overlapping by hand.
+__device__ __forceinline__ void grid_dependency_begin() {
+  ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // 16-byte vector of T.
 template <typename T> struct Vec16 {
   static constexpr int N = 16 / sizeof(T);
@@ -101,6 +134,17 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   }
   __syncthreads();
   return red[32];
+}
+
+// The same sum with one barrier instead of two: every warp adds up the warps' sums itself.  `red` must not be written
+// again before a barrier.
+__device__ __forceinline__ float block_sum_once(float v, float* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = warp_sum(v);
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  const int nw = (blockDim.x + 31) >> 5;
+  return warp_sum(lane < nw ? red[lane] : 0.f);
 }
 
 __host__ __device__ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

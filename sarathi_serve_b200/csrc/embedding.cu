@@ -13,6 +13,7 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 vocab_embedding_kernel(T* __restrict__ out, const int64_t* __restrict__ ids, const T* __restrict__ weight, int64_t T_,
                        int64_t H, int64_t vocab_start, int64_t vocab_end) {
+  grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t i_first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -61,9 +62,9 @@ static int launch_vocab_embedding(void* out, const int64_t* ids, const void* wei
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   if (vec)
-    vocab_embedding_kernel<T, true><<<(int)blocks, 256, 0, s>>>((T*)out, ids, (const T*)weight, T_, H, v0, v1);
+    launch_dependent(vocab_embedding_kernel<T, true>, (int)blocks, 256, 0, s, (T*)out, ids, (const T*)weight, T_, H, v0, v1);
   else
-    vocab_embedding_kernel<T, false><<<(int)blocks, 256, 0, s>>>((T*)out, ids, (const T*)weight, T_, H, v0, v1);
+    launch_dependent(vocab_embedding_kernel<T, false>, (int)blocks, 256, 0, s, (T*)out, ids, (const T*)weight, T_, H, v0, v1);
   SB_CHECK_LAUNCH("vocab_embedding_kernel");
   return SB200_OK;
 }

@@ -263,18 +263,6 @@ uint32_t gemm_push_increments(const GemmPlan& p, int64_t M, int64_t lo, int64_t 
   return (uint32_t)total;
 }
 
-// Programmatic dependent launch of the GEMM kernels: off unless SB200_PDL=1.  Measured on the TP=1 layer
-// step it gains about 1 us of 244 (only GEMM -> GEMM boundaries overlap, and a CTA of the next kernel cannot
-// become resident before a CTA of this one has left its SM), so it is not worth a default.
-static bool pdl_enabled() {
-  static int v = -1;
-  if (v < 0) {
-    const char* e = getenv("SB200_PDL");
-    v = (e && atoi(e) != 0) ? 1 : 0;
-  }
-  return v != 0;
-}
-
 // Distance (k-blocks) of the L2 prefetch of weight boxes; SB200_L2_PREFETCH overrides (0 disables).
 static int l2_prefetch_distance() {
   static int v = -1;
@@ -287,7 +275,7 @@ static int l2_prefetch_distance() {
 }
 
 template <typename T, int EPI, bool CTA2, int MI>
-static int launch_sm100(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, const CommView& cv,
+static int launch_sm100(const CUtensorMap& ta, const CUtensorMap& tat, const CUtensorMap& tb, const GemmArgs& g, const CommView& cv,
                         const ReduceArgs& ra, cudaStream_t s) {
   auto kern = gemm_sm100_kernel<T, EPI, CTA2, MI>;
   static thread_local int configured_dev = -1;
@@ -312,31 +300,32 @@ static int launch_sm100(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   // programmatic dependent launch: the prologue (barriers, TMEM, tensor maps) may run while the previous
-  // kernel of the stream finishes; the kernel waits for it before its first global access
+  // kernel of the stream finishes; the kernel waits for it before its first global access.  Not for the
+  // row-parallel kernel: its CTAs wait for other ranks, and nothing else should sit on an SM meanwhile.
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  SB_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, g, cv, ra));
+  cfg.numAttrs = EPI == EPI_PUSH ? 1 : 2;
+  SB_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tat, tb, g, cv, ra));
   return SB200_OK;
 }
 
 template <typename T, int EPI>
-static int launch_mode(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, const CommView& cv,
+static int launch_mode(const CUtensorMap& ta, const CUtensorMap& tat, const CUtensorMap& tb, const GemmArgs& g, const CommView& cv,
                        const ReduceArgs& ra, cudaStream_t s) {
-  if (g.cta2) return g.mi == 2 ? launch_sm100<T, EPI, true, 2>(ta, tb, g, cv, ra, s) : launch_sm100<T, EPI, true, 1>(ta, tb, g, cv, ra, s);
-  return g.mi == 2 ? launch_sm100<T, EPI, false, 2>(ta, tb, g, cv, ra, s) : launch_sm100<T, EPI, false, 1>(ta, tb, g, cv, ra, s);
+  if (g.cta2) return g.mi == 2 ? launch_sm100<T, EPI, true, 2>(ta, tat, tb, g, cv, ra, s) : launch_sm100<T, EPI, true, 1>(ta, tat, tb, g, cv, ra, s);
+  return g.mi == 2 ? launch_sm100<T, EPI, false, 2>(ta, tat, tb, g, cv, ra, s) : launch_sm100<T, EPI, false, 1>(ta, tat, tb, g, cv, ra, s);
 }
 
 template <typename T>
-static int dispatch_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g,
+static int dispatch_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tat, const CUtensorMap& tb, const GemmArgs& g,
                         const CommView& cv, const ReduceArgs& ra, cudaStream_t s) {
   switch (epi) {
-    case EPI_STORE: return launch_mode<T, EPI_STORE>(ta, tb, g, cv, ra, s);
-    case EPI_ROTARY: return launch_mode<T, EPI_ROTARY>(ta, tb, g, cv, ra, s);
-    case EPI_SILU_MUL: return launch_mode<T, EPI_SILU_MUL>(ta, tb, g, cv, ra, s);
-    case EPI_PUSH: return launch_mode<T, EPI_PUSH>(ta, tb, g, cv, ra, s);
-    case EPI_MOE_SCATTER: return launch_mode<T, EPI_MOE_SCATTER>(ta, tb, g, cv, ra, s);
+    case EPI_STORE: return launch_mode<T, EPI_STORE>(ta, tat, tb, g, cv, ra, s);
+    case EPI_ROTARY: return launch_mode<T, EPI_ROTARY>(ta, tat, tb, g, cv, ra, s);
+    case EPI_SILU_MUL: return launch_mode<T, EPI_SILU_MUL>(ta, tat, tb, g, cv, ra, s);
+    case EPI_PUSH: return launch_mode<T, EPI_PUSH>(ta, tat, tb, g, cv, ra, s);
+    case EPI_MOE_SCATTER: return launch_mode<T, EPI_MOE_SCATTER>(ta, tat, tb, g, cv, ra, s);
   }
   set_error("unknown GEMM epilogue %d", epi);
   return SB200_ERR_INVALID_ARGUMENT;
@@ -357,15 +346,20 @@ int run_gemm_sm100(int dtype, int epi, const GemmPlan& plan, const void* x, int6
     g.ws_counters = reinterpret_cast<uint32_t*>(workspace);
     g.ws = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + kWsCounterBytes);
   }
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tat, tb;
   int rc = make_tmap_2d(&ta, dtype, x, g.M, g.K, ldx, 128, kBK);
   if (rc) return rc;
+  tat = ta;
+  if (g.M % 128) {
+    rc = make_tmap_2d(&tat, dtype, x, g.M, g.K, ldx, a_box_rows(g.M % 128), kBK);
+    if (rc) return rc;
+  }
   g.rot_split = (epi == EPI_ROTARY && plan.bn < g.head_size) ? 1 : 0;
   rc = make_tmap_2d(&tb, dtype, w, b_rows > 0 ? b_rows : g.N, g.K, ldw,
                     (epi == EPI_SILU_MUL || plan.cta2 || g.rot_split) ? plan.bn / 2 : plan.bn, kBK);
   if (rc) return rc;
-  if (dtype == SB200_BF16) return dispatch_epi<__nv_bfloat16>(epi, ta, tb, g, cv, ra, s);
-  if (dtype == SB200_F16) return dispatch_epi<__half>(epi, ta, tb, g, cv, ra, s);
+  if (dtype == SB200_BF16) return dispatch_epi<__nv_bfloat16>(epi, ta, tat, tb, g, cv, ra, s);
+  if (dtype == SB200_F16) return dispatch_epi<__half>(epi, ta, tat, tb, g, cv, ra, s);
   set_error("tcgen05 GEMM supports bf16/fp16 only");
   return SB200_ERR_UNSUPPORTED;
 }

@@ -83,8 +83,9 @@ gemm_f32_kernel(float* __restrict__ C, int64_t ldc, const float* __restrict__ A,
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * kF32BN;
   const int S = gridDim.z, part = blockIdx.z;
   const int kt_all = (K + kF32BK - 1) / kF32BK;
-  const int kt0 = (int)((int64_t)kt_all * part / S), kt1 = (int)((int64_t)kt_all * (part + 1) / S);
+  const int kt0 = (int)((unsigned)kt_all * (unsigned)part / (unsigned)S), kt1 = (int)((unsigned)kt_all * (unsigned)(part + 1) / (unsigned)S);
   const int lrow = tid >> 2, lk = (tid & 3) * 4;
+  grid_dependency_begin();
 
   unsigned long long acc[TM][4];
 #pragma unroll
@@ -220,13 +221,15 @@ static int launch_f32(float* C, int64_t ldc, const float* A, int64_t lda, const 
   cfg.gridDim = dim3((unsigned)nt, (unsigned)mt, (unsigned)split);
   cfg.blockDim = dim3(kF32Threads);
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = (unsigned)split;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   if (vec) SB_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<BM, true>, C, ldc, A, lda, B, ldb, bias, M, N, K, vec_c));
   else SB_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<BM, false>, C, ldc, A, lda, B, ldb, bias, M, N, K, vec_c));
   return SB200_OK;

@@ -38,7 +38,7 @@
 // Grouped (mixture-of-experts) mode: when `expert_ids` is set, the rows of A are the
 // expert-sorted, block-padded slots of moe_align_block_size (block = tile rows), tile row block
 // mt uses the weights of expert expert_ids[mt] (B rows offset by expert * rows_per_expert), and
-// row blocks at or beyond *num_post_pad are skipped.
+// row blocks at or beyond *num_post_pad have no tiles.
 #pragma once
 
 #include "comm.cuh"
@@ -118,6 +118,9 @@ struct GemmArgs {
                            // 1.. travel to pair 0 through distributed shared memory and pair 0 runs the epilogue
   uint32_t* status;        // device word: first error of this launch (0 = none); may be null
 };
+
+// Rows of the A box of a 128-row accumulator block that has `left` rows of the matrix from its first one on.
+__host__ __device__ inline int a_box_rows(int left) { return left >= 128 ? 128 : left <= 0 ? 0 : (left + 7) & ~7; }
 
 // Shared memory of one pipeline stage in one CTA (a CTA of a pair keeps half of the B tile).
 __host__ __device__ inline int gemm_stage_bytes(int mi, int bn, int cta2 = 0) {
@@ -603,7 +606,8 @@ __device__ __forceinline__ void push_rows_done(const CommView& comm, const Reduc
 //                 accumulator rows.  Per SM this halves the shared-memory traffic of the B operand.
 template <typename T, int EPI, bool CTA2, int MI>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_at,
+                  const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ GemmArgs g, const __grid_constant__ CommView comm,
                   const __grid_constant__ ReduceArgs red) {
   constexpr uint32_t kTmemCols = 512;
@@ -642,7 +646,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   // each epilogue warp's block for the transposing stores (warps 0 and 1 never use theirs)
   uint8_t* epi_stage = smem + (size_t)kStages * stage_bytes + kBarrierBytes + (size_t)((threadIdx.x >> 5) >= 2 ? (threadIdx.x >> 5) - 2 : 0) * kEpiWarpStageBytes;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (read from lane 0, so that the compiler knows the role branches and the epilogue's loops to be warp-uniform: they
+  // hold instructions that all lanes have to execute together)
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 #ifdef SB200_TRACE
   __shared__ unsigned int gemm_trace_row_s;
   if (blockIdx.x == 0 && threadIdx.x == 0) gemm_trace_row_s = atomicAdd(&g_gemm_trace_launch, 1u);
@@ -658,10 +664,6 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   sc.Gs = g.rem_units;
   sc.k_blocks = g.k_blocks;
   sc.rounds = g.tiles_full / num_units_grid;
-  // Every CTA of this persistent grid is resident from the start, so the next kernel of the stream may be
-  // scheduled onto SMs as they become free (its prologue then overlaps this kernel's tail).
-  ptx::grid_launch_dependents();
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(&full_bar[s], 1);
@@ -677,6 +679,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
   if (warp == 0 && lane == 0) {
     ptx::prefetch_tensormap(&tmap_a);
+    ptx::prefetch_tensormap(&tmap_at);
     ptx::prefetch_tensormap(&tmap_b);
   }
   if (warp == 1) {
@@ -688,6 +691,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   if (CTA2) ptx::cluster_sync_all();  // the peer's barriers are initialised before anything signals them
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Every CTA of this persistent grid is resident from the start, so the next kernel of the stream may be
+  // scheduled onto SMs as they become free (its prologue then overlaps this kernel's tail).
+  if constexpr (EPI != EPI_PUSH) ptx::grid_launch_dependents();
 #ifdef SB200_TRACE
   gemm_trace_row = gemm_trace_row_s;
   if (threadIdx.x == 0) SB_GEMM_MARK(1);  // prologue done
@@ -696,79 +702,105 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   ptx::grid_dependency_wait();
   if (threadIdx.x == 0) SB_GEMM_MARK(10);  // after the dependency wait
   // grouped mode: rows of A in use (a device value written by moe_align_block_size earlier in the stream)
-  const int rows_in_use = g.expert_ids ? min(g.M, *g.num_post_pad) : g.M;
+  // and the tiles that have any.  They are dealt out by their number in use, so that skipped row blocks leave no unit
+  // with fewer tiles than the others (all tiles are whole in this mode).
+  int m_tiles = g.m_tiles;
+  if (g.expert_ids) {
+    m_tiles = (min(g.M, *g.num_post_pad) + BM - 1) / BM;
+    const int tiles = m_tiles * g.n_tiles;
+    sc.rounds = tiles / num_units_grid;
+    sc.tiles_full = sc.rounds * num_units_grid;
+    sc.rem_tiles = sc.Gs = tiles - sc.tiles_full;
+  }
 
+  __syncwarp();  // the roles start from converged warps
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (ptx::elect_one()) {
+    {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      SB_GEMM_MARK(14);  // producer entered
+      if (lane == 0) SB_GEMM_MARK(14);  // producer entered
       for (int it = 0; ok; ++it) {
         const Segment sg = segment_of(sc, unit_id, it);
         if (!sg.valid) break;
-        if (it == 0) SB_GEMM_MARK(15);  // first segment known
-        const int mt = sg.tile % g.m_tiles, nt = sg.tile / g.m_tiles;
+        if (it == 0 && lane == 0) SB_GEMM_MARK(15);  // first segment known
+        const int mt = sg.tile % m_tiles, nt = sg.tile / m_tiles;
         int b_row0 = 0;  // grouped mode: first B row of this row block's expert
-        if (g.expert_ids) {
-          if (mt * BM >= rows_in_use) continue;  // row block beyond the padded slots: every role skips it
-          b_row0 = g.expert_ids[mt] * g.rows_per_expert;
+        if (g.expert_ids) b_row0 = g.expert_ids[mt] * g.rows_per_expert;
+        // Rows of A this CTA loads per accumulator: a 128-row box, or the shorter box of `tmap_at` for the last,
+        // partial one, or none.  (The rows of a box that lie outside the tensor are not free: with 8 tokens in a
+        // 128-row box a k-block took 0.85 us, with 64 tokens 0.7 us.  Rows that are not loaded hold whatever the
+        // stage held before; they only reach accumulator rows that are never stored.)
+        int a_rows[MI];
+        uint32_t tx_bytes = (uint32_t)((CTA2 ? 2 : 1) * b_rows * kBK * 2);  // (a pair's leader announces both CTAs' bytes)
+#pragma unroll
+        for (int a = 0; a < MI; ++a) {
+          a_rows[a] = a_box_rows(g.M - (mt * BM + a * (CTA2 ? 256 : 128) + (int)cta_rank * 128));
+          tx_bytes += (uint32_t)(a_rows[a] * kBK * 2);
+          if (CTA2) tx_bytes += (uint32_t)(a_box_rows(g.M - (mt * BM + a * 256 + (int)(cta_rank ^ 1u) * 128)) * kBK * 2);
         }
         const int p_kb1 = kb_hi(sg);
         for (int kb = kb_lo(sg); kb < p_kb1; ++kb) {
-          if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          if (kb == kb_lo(sg) && it == 0) SB_GEMM_MARK(11);  // stage 0 free, about to request it
-          uint8_t* sa = stage_base + (size_t)stage * stage_bytes;
-          uint8_t* sb = sa + a_bytes;
-          const bool halves = (EPI == EPI_SILU_MUL) || (EPI == EPI_ROTARY && g.rot_split);  // B tile = two row blocks
-          const int b_first = tile_first_col<EPI>(g, nt);                                  // first row of the first block
-          const int b_second = b_first + (EPI == EPI_SILU_MUL ? g.N / 2 : g.head_size / 2);  // ... of the second
-          if (g.l2_prefetch > 0 && kb + g.l2_prefetch < p_kb1 && !(EPI == EPI_ROTARY && g.rot_split)) {
-            // weights are read once: start their trip from HBM to L2 a few stages early
-            const int pk = (kb + g.l2_prefetch) * kBK;
-            if (CTA2) {
-              ptx::tma_prefetch_l2_2d(&tmap_b, pk, (EPI == EPI_SILU_MUL) ? (int)cta_rank * (g.N / 2) + nt * (BN / 2)
-                                                                        : nt * BN + (int)cta_rank * (BN / 2));
+          if (!ptx::mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+          if (kb == kb_lo(sg) && it == 0 && lane == 0) SB_GEMM_MARK(11);  // stage 0 free, about to request it
+          if (ptx::elect_one()) {
+            uint8_t* sa = stage_base + (size_t)stage * stage_bytes;
+            uint8_t* sb = sa + a_bytes;
+            const bool halves = (EPI == EPI_SILU_MUL) || (EPI == EPI_ROTARY && g.rot_split);  // B tile = two row blocks
+            const int b_first = tile_first_col<EPI>(g, nt);                                  // first row of the first block
+            const int b_second = b_first + (EPI == EPI_SILU_MUL ? g.N / 2 : g.head_size / 2);  // ... of the second
+            if (g.l2_prefetch > 0 && kb + g.l2_prefetch < p_kb1 && !(EPI == EPI_ROTARY && g.rot_split)) {
+              // weights are read once: start their trip from HBM to L2 a few stages early
+              const int pk = (kb + g.l2_prefetch) * kBK;
+              if (CTA2) {
+                ptx::tma_prefetch_l2_2d(&tmap_b, pk, (EPI == EPI_SILU_MUL) ? (int)cta_rank * (g.N / 2) + nt * (BN / 2)
+                                                                          : nt * BN + (int)cta_rank * (BN / 2));
+              } else {
+                ptx::tma_prefetch_l2_2d(&tmap_b, pk, (EPI == EPI_SILU_MUL) ? nt * (BN / 2) : nt * BN);
+                if (EPI == EPI_SILU_MUL) ptx::tma_prefetch_l2_2d(&tmap_b, pk, g.N / 2 + nt * (BN / 2));
+              }
+            }
+            if constexpr (CTA2) {
+              // both CTAs' bytes are counted on the leader's barrier; only the leader announces them
+              const uint32_t bar = ptx::map_to_cta(ptx::smem_u32(&full_bar[stage]), pair_base);
+              if (leader) ptx::mbar_expect_tx(&full_bar[stage], tx_bytes);
+#pragma unroll
+              for (int a = 0; a < MI; ++a)  // accumulator a covers tile rows [256a, 256a+256): this CTA's half of them
+                if (a_rows[a] > 0)
+                  ptx::tma_load_2d_pair(sa + a * (128 * kBK * 2), a_rows[a] == 128 ? &tmap_a : &tmap_at, bar, kb * kBK,
+                                        mt * BM + a * 256 + (int)cta_rank * 128);
+              if (halves)  // even CTA: gate rows (first half of the head), odd CTA: the matching up rows (second half)
+                ptx::tma_load_2d_pair(sb, &tmap_b, bar, kb * kBK, b_row0 + (cta_rank ? b_second : b_first));
+              else
+                ptx::tma_load_2d_pair(sb, &tmap_b, bar, kb * kBK, b_row0 + nt * BN + (int)cta_rank * (BN / 2));
             } else {
-              ptx::tma_prefetch_l2_2d(&tmap_b, pk, (EPI == EPI_SILU_MUL) ? nt * (BN / 2) : nt * BN);
-              if (EPI == EPI_SILU_MUL) ptx::tma_prefetch_l2_2d(&tmap_b, pk, g.N / 2 + nt * (BN / 2));
+              ptx::mbar_expect_tx(&full_bar[stage], tx_bytes);
+#pragma unroll
+              for (int a = 0; a < MI; ++a)
+                if (a_rows[a] > 0)
+                  ptx::tma_load_2d(sa + a * (128 * kBK * 2), a_rows[a] == 128 ? &tmap_a : &tmap_at, &full_bar[stage], kb * kBK,
+                                   mt * BM + a * 128);
+              if (halves) {
+                // B tile = BN/2 rows of the gate shard followed by the matching BN/2 rows of the up shard
+                // (rotary: of the first and of the second half of the head)
+                ptx::tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * kBK, b_row0 + b_first);
+                ptx::tma_load_2d(sb + (BN / 2) * (kBK * 2), &tmap_b, &full_bar[stage], kb * kBK, b_row0 + b_second);
+              } else {
+                ptx::tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * kBK, b_row0 + nt * BN);
+              }
             }
           }
-          if constexpr (CTA2) {
-            // both CTAs' bytes are counted on the leader's barrier; only the leader announces them
-            const uint32_t bar = ptx::map_to_cta(ptx::smem_u32(&full_bar[stage]), pair_base);
-            if (leader) ptx::mbar_expect_tx(&full_bar[stage], (uint32_t)(2 * stage_bytes));
-#pragma unroll
-            for (int a = 0; a < MI; ++a)  // accumulator a covers tile rows [256a, 256a+256): this CTA's half of them
-              ptx::tma_load_2d_pair(sa + a * (128 * kBK * 2), &tmap_a, bar, kb * kBK, mt * BM + a * 256 + (int)cta_rank * 128);
-            if (halves)  // even CTA: gate rows (first half of the head), odd CTA: the matching up rows (second half)
-              ptx::tma_load_2d_pair(sb, &tmap_b, bar, kb * kBK, b_row0 + (cta_rank ? b_second : b_first));
-            else
-              ptx::tma_load_2d_pair(sb, &tmap_b, bar, kb * kBK, b_row0 + nt * BN + (int)cta_rank * (BN / 2));
-          } else {
-            ptx::mbar_expect_tx(&full_bar[stage], (uint32_t)stage_bytes);
-#pragma unroll
-            for (int a = 0; a < MI; ++a)
-              ptx::tma_load_2d(sa + a * (128 * kBK * 2), &tmap_a, &full_bar[stage], kb * kBK, mt * BM + a * 128);
-            if (halves) {
-              // B tile = BN/2 rows of the gate shard followed by the matching BN/2 rows of the up shard
-              // (rotary: of the first and of the second half of the head)
-              ptx::tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * kBK, b_row0 + b_first);
-              ptx::tma_load_2d(sb + (BN / 2) * (kBK * 2), &tmap_b, &full_bar[stage], kb * kBK, b_row0 + b_second);
-            } else {
-              ptx::tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * kBK, b_row0 + nt * BN);
-            }
-          }
-          if (kb == kb_lo(sg) && it == 0) SB_GEMM_MARK(2);  // first stage requested
+          __syncwarp();
+          if (kb == kb_lo(sg) && it == 0 && lane == 0) SB_GEMM_MARK(2);  // first stage requested
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
-      SB_GEMM_MARK(3);  // last stage requested
+      if (lane == 0) SB_GEMM_MARK(3);  // last stage requested
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (leader && ptx::elect_one()) {
+    if (leader) {
       int stage = 0;
       uint32_t phase = 0;
       int used = 0;  // tiles actually computed (selects the TMEM buffer)
@@ -776,39 +808,42 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       for (int it = 0; ok; ++it) {
         const Segment sg = segment_of(sc, unit_id, it);
         if (!sg.valid) break;
-        if (g.expert_ids && (sg.tile % g.m_tiles) * BM >= rows_in_use) continue;
         const int local = used++;
         const int kb0 = kb_lo(sg), kb1 = kb_hi(sg);
         const int buf = dbuf ? (local & 1) : 0;
         const uint32_t use = (uint32_t)(dbuf ? (local >> 1) : local);  // earlier uses of this buffer
-        if (!ptx::mbar_wait(&tmem_empty[buf], (use & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+        if (!ptx::mbar_wait_warp(&tmem_empty[buf], (use & 1u) ^ 1u, abort_flag)) { ok = false; break; }
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * MI * BN);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!ptx::mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+          if (!ptx::mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after();
-          if (kb == kb0 && it == 0) SB_GEMM_MARK(4);  // first stage arrived
-          const uint32_t sa = ptx::smem_u32(stage_base + (size_t)stage * stage_bytes);
-          const uint64_t db = ptx::make_smem_desc_sw128(sa + a_bytes);
+          if (kb == kb0 && it == 0 && lane == 0) SB_GEMM_MARK(4);  // first stage arrived
+          if (ptx::elect_one()) {
+            const uint32_t sa = ptx::smem_u32(stage_base + (size_t)stage * stage_bytes);
+            const uint64_t db = ptx::make_smem_desc_sw128(sa + a_bytes);
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) {
-            // advance 16 elements = 32 bytes along K inside the swizzle row: +2 in 16-byte units
-            const uint32_t acc = (kb > kb0 || k > 0) ? 1u : 0u;
+            for (int k = 0; k < kBK / 16; ++k) {
+              // advance 16 elements = 32 bytes along K inside the swizzle row: +2 in 16-byte units
+              const uint32_t acc = (kb > kb0 || k > 0) ? 1u : 0u;
 #pragma unroll
-            for (int a = 0; a < MI; ++a) {
-              const uint64_t da = ptx::make_smem_desc_sw128(sa + a * (128 * kBK * 2));
-              if (CTA2) ptx::umma_f16_pair(d_tmem + (uint32_t)(a * BN), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, acc);
-              else ptx::umma_f16(d_tmem + (uint32_t)(a * BN), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, acc);
+              for (int a = 0; a < MI; ++a) {
+                const uint64_t da = ptx::make_smem_desc_sw128(sa + a * (128 * kBK * 2));
+                if (CTA2) ptx::umma_f16_pair(d_tmem + (uint32_t)(a * BN), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, acc);
+                else ptx::umma_f16(d_tmem + (uint32_t)(a * BN), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, acc);
+              }
             }
+            // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
+            if (CTA2) ptx::umma_commit_pair_mask(&empty_bar[stage], pair_mask); else ptx::umma_commit(&empty_bar[stage]);
           }
-          // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
-          if (CTA2) ptx::umma_commit_pair_mask(&empty_bar[stage], pair_mask); else ptx::umma_commit(&empty_bar[stage]);
+          __syncwarp();
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
-        if (ok) {  // accumulators complete
+        if (ok && ptx::elect_one()) {  // accumulators complete (the same lane: a commit covers what its thread issued)
           if (CTA2) ptx::umma_commit_pair_mask(&tmem_full[buf], pair_mask); else ptx::umma_commit(&tmem_full[buf]);
         }
-        SB_GEMM_MARK(5);  // last MMA issued
+        __syncwarp();
+        if (lane == 0) SB_GEMM_MARK(5);  // last MMA issued
       }
     }
   } else {
@@ -827,13 +862,13 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const Segment sg = segment_of(sc, unit_id, it);
       if (!sg.valid) break;
       const int tile = sg.tile, S = sg.parts;
-      const int mt = tile % g.m_tiles, nt = tile / g.m_tiles;
-      if (g.expert_ids && mt * BM >= rows_in_use) continue;
+      const int mt = tile % m_tiles, nt = tile / m_tiles;
       const int local = used++;
       const int buf = dbuf ? (local & 1) : 0;
       const uint32_t use = (uint32_t)(dbuf ? (local >> 1) : local);
       ok = __all_sync(0xffffffffu, ptx::mbar_wait(&tmem_full[buf], use & 1u, abort_flag) ? 1 : 0) != 0;
       if (!ok) break;  // warp-uniform: no lane is left behind in an aligned tcgen05.ld
+      __syncwarp();
       ptx::tc_fence_after();
       if (warp == 2 && lane == 0) SB_GEMM_MARK(6);  // accumulators complete (seen by the epilogue)
 
@@ -883,8 +918,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       if (!sg.valid) break;
       const int S = sg.parts;
       if (S == 1) continue;
-      const int mt = sg.tile % g.m_tiles, nt = sg.tile / g.m_tiles;
-      if (g.expert_ids && mt * BM >= rows_in_use) continue;
+      const int mt = sg.tile % m_tiles, nt = sg.tile / m_tiles;
       uint32_t* ctr_arrive = g.ws_counters + (size_t)sg.rem_index * 32 + slot;
       uint32_t* ctr_done = ctr_arrive + 16;
       int arrived = 1;

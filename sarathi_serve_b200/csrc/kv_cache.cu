@@ -23,6 +23,7 @@ namespace sb200 {
 __global__ void kv_slots_kernel(int64_t* __restrict__ slots, const int32_t* __restrict__ batch_indices,
                                 const int32_t* __restrict__ positions, const int32_t* __restrict__ kv_indices,
                                 const int32_t* __restrict__ kv_indptr, int64_t n, int page_size) {
+  grid_dependency_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int b = batch_indices[i];
@@ -36,6 +37,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 kv_append_kernel(T* __restrict__ cache, const T* __restrict__ k, int64_t ldk, const T* __restrict__ v, int64_t ldv,
                  const int64_t* __restrict__ slots, int64_t n, int row_elems, int page_size) {
+  grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int nvec = row_elems / N;
   const int64_t total = n * nvec * 2, stride = (int64_t)gridDim.x * blockDim.x;
@@ -60,7 +62,7 @@ extern "C" int sb200_kv_cache_slots(int64_t* slots, const int32_t* batch_indices
   SB_CHECK_ARG(n >= 0 && page_size > 0, "kv_cache_slots: bad sizes");
   if (n == 0) return SB200_OK;
   SB_CHECK_ARG(slots && batch_indices && positions && kv_indices && kv_indptr, "kv_cache_slots: null pointer");
-  kv_slots_kernel<<<(int)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(slots, batch_indices, positions, kv_indices,
+  launch_dependent(kv_slots_kernel, (int)((n + 255) / 256), 256, 0, (cudaStream_t)stream, slots, batch_indices, positions, kv_indices,
                                                                             kv_indptr, n, page_size);
   SB_CHECK_LAUNCH("kv_slots_kernel");
   return SB200_OK;
@@ -80,7 +82,7 @@ extern "C" int sb200_kv_cache_append(void* cache, const void* k, int64_t ldk, co
   int64_t blocks = (n * 2 * (row / (16 / (int64_t)es)) + 255) / 256;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  SB_DISPATCH_FLOAT(dtype, (kv_append_kernel<scalar_t><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(
+  SB_DISPATCH_FLOAT(dtype, (launch_dependent(kv_append_kernel<scalar_t>, (int)blocks, 256, 0, (cudaStream_t)stream, 
                                (scalar_t*)cache, (const scalar_t*)k, ldk, (const scalar_t*)v, ldv, slots, n, (int)row,
                                page_size)));
   SB_CHECK_LAUNCH("kv_append_kernel");

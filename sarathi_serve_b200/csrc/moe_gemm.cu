@@ -17,6 +17,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(T* __restrict__ out, const T* __restrict__ x, const int32_t* __restrict__ sorted_ids,
                   const int32_t* __restrict__ num_post_pad, int64_t rows_cap, int64_t num_slots, int H, int top_k) {
+  grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int nvec = H / N;
   const int64_t rows = min((int64_t)*num_post_pad, rows_cap);
@@ -36,6 +37,7 @@ moe_gather_kernel(T* __restrict__ out, const T* __restrict__ x, const int32_t* _
 template <typename T>
 __global__ void __launch_bounds__(256)
 moe_sum_kernel(T* __restrict__ out, const T* __restrict__ in3, const T* __restrict__ residual, int64_t T_, int k, int H) {
+  grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int nvec = H / N;
   const int64_t total = T_ * nvec, stride = (int64_t)gridDim.x * blockDim.x;
@@ -121,7 +123,7 @@ extern "C" int sb200_moe_gather_rows(void* out, const void* x, const int32_t* so
   if (rows_cap == 0) return SB200_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const int grid = grid_1d(rows_cap * (H / (16 / (int64_t)dtype_size(dtype))));
-  SB_DISPATCH_FLOAT(dtype, (moe_gather_kernel<scalar_t><<<grid, 256, 0, s>>>((scalar_t*)out, (const scalar_t*)x, sorted_ids,
+  SB_DISPATCH_FLOAT(dtype, (launch_dependent(moe_gather_kernel<scalar_t>, grid, 256, 0, s, (scalar_t*)out, (const scalar_t*)x, sorted_ids,
                                                                             num_post_pad, rows_cap, T * top_k, (int)H, top_k)));
   SB_CHECK_LAUNCH("moe_gather_kernel");
   return SB200_OK;
@@ -152,7 +154,7 @@ extern "C" int sb200_moe_sum(void* out, const void* in3, const void* residual, i
   if (T == 0) return SB200_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const int grid = grid_1d(T * (H / (16 / (int64_t)dtype_size(dtype))));
-  SB_DISPATCH_FLOAT(dtype, (moe_sum_kernel<scalar_t><<<grid, 256, 0, s>>>((scalar_t*)out, (const scalar_t*)in3,
+  SB_DISPATCH_FLOAT(dtype, (launch_dependent(moe_sum_kernel<scalar_t>, grid, 256, 0, s, (scalar_t*)out, (const scalar_t*)in3,
                                                                          (const scalar_t*)residual, T, top_k, (int)H)));
   SB_CHECK_LAUNCH("moe_sum_kernel");
   return SB200_OK;

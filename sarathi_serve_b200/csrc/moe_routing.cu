@@ -41,6 +41,7 @@ template <int E, typename TIn, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 topk_softmax_pow2_kernel(const TIn* __restrict__ gating, float* __restrict__ weights, int32_t* __restrict__ ids,
                          int32_t* __restrict__ src_rows, int64_t num_rows, int k, int renorm) {
+  grid_dependency_begin();
   using L = TopkLayout<E>;
   constexpr int VPT = L::VPT, TPR = L::TPR, EPL = L::ELTS_PER_LDG, LDGS = L::VECS;
   constexpr int COLS_PER_GROUP = EPL * TPR;
@@ -116,6 +117,7 @@ template <typename TIn>
 __global__ void __launch_bounds__(256)
 topk_softmax_generic_kernel(const TIn* __restrict__ gating, float* __restrict__ weights, int32_t* __restrict__ ids,
                             int32_t* __restrict__ src_rows, int64_t num_rows, int E, int k, int renorm) {
+  grid_dependency_begin();
   constexpr int TPB = 256;
   using BlockReduce = cub::BlockReduce<float, TPB>;
   __shared__ typename BlockReduce::TempStorage tmp;
@@ -178,7 +180,7 @@ static void launch_topk_pow2(const void* g, float* w, int32_t* ids, int32_t* src
   constexpr int WARPS = 4;
   const int64_t rows_per_cta = WARPS * TopkLayout<E>::ROWS_PER_WARP;
   const int64_t blocks = (T_ + rows_per_cta - 1) / rows_per_cta;
-  topk_softmax_pow2_kernel<E, TIn, WARPS><<<(unsigned)blocks, WARPS * 32, 0, s>>>((const TIn*)g, w, ids, src, T_, k, renorm);
+  launch_dependent(topk_softmax_pow2_kernel<E, TIn, WARPS>, (unsigned)blocks, WARPS * 32, 0, s, (const TIn*)g, w, ids, src, T_, k, renorm);
 }
 
 template <typename TIn>
@@ -196,7 +198,7 @@ static int launch_topk(const void* g, float* w, int32_t* ids, int32_t* src, int6
       }
       if (smem > 40 * 1024)
         SB_CUDA(cudaFuncSetAttribute(topk_softmax_generic_kernel<TIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      topk_softmax_generic_kernel<TIn><<<(unsigned)T_, 256, smem, s>>>((const TIn*)g, w, ids, src, T_, E, k, renorm);
+      launch_dependent(topk_softmax_generic_kernel<TIn>, (unsigned)T_, 256, smem, s, (const TIn*)g, w, ids, src, T_, E, k, renorm);
     }
   }
   SB_CHECK_LAUNCH("topk_softmax kernel");
@@ -262,6 +264,7 @@ __device__ __forceinline__ int find_expert(const int* cumsum, int E, int pos) {
 __global__ void __launch_bounds__(1024)
 moe_align_single_kernel(const void* ids, int itype, int64_t numel, int E, int block, int32_t* sorted,
                         int64_t sorted_cap, int32_t* expert_ids, int64_t expert_cap, int32_t* num_post_pad) {
+  grid_dependency_begin();
   extern __shared__ int sm[];
   int* cnt = sm;                 // [32][E]
   int* cumsum = sm + 32 * E;     // [E+1]
@@ -301,6 +304,7 @@ moe_align_single_kernel(const void* ids, int itype, int64_t numel, int E, int bl
 __global__ void __launch_bounds__(256)
 moe_align_count_kernel(const void* ids, int itype, int64_t numel, int E, int64_t seg_len, int nseg, int* scratch,
                        int32_t* sorted, int64_t sorted_cap) {
+  grid_dependency_begin();
   const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gsz = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = gtid; i < sorted_cap; i += gsz) sorted[i] = (int32_t)numel;
   const int seg = (int)(gtid >> 5);
@@ -316,6 +320,7 @@ moe_align_count_kernel(const void* ids, int itype, int64_t numel, int E, int64_t
 __global__ void __launch_bounds__(1024)
 moe_align_scan_kernel(int E, int block, int nseg, int* scratch, int32_t* expert_ids, int64_t expert_cap,
                       int32_t* num_post_pad) {
+  grid_dependency_begin();
   int* cumsum = scratch + (int64_t)nseg * E;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int e = warp; e < E; e += 32) {
@@ -348,6 +353,7 @@ moe_align_scan_kernel(int E, int block, int nseg, int* scratch, int32_t* expert_
 __global__ void __launch_bounds__(256)
 moe_align_scatter_kernel(const void* ids, int itype, int64_t numel, int E, int64_t seg_len, int nseg, int* scratch,
                          int32_t* sorted) {
+  grid_dependency_begin();
   const int seg = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (seg >= nseg) return;
   const int64_t lo = min((int64_t)seg * seg_len, numel), hi = min(lo + seg_len, numel);
@@ -419,7 +425,7 @@ extern "C" int sb200_moe_align_block_size(const void* topk_ids, int ids_itype, i
     }
     if (smem > 40 * 1024)
       SB_CUDA(cudaFuncSetAttribute(moe_align_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    moe_align_single_kernel<<<1, 1024, smem, s>>>(topk_ids, ids_itype, numel, E, block_size, sorted_token_ids,
+    launch_dependent(moe_align_single_kernel, 1, 1024, smem, s, topk_ids, ids_itype, numel, E, block_size, sorted_token_ids,
                                                   sorted_capacity, expert_ids, expert_ids_capacity,
                                                   num_tokens_post_pad);
     SB_CHECK_LAUNCH("moe_align_single_kernel");
@@ -427,13 +433,13 @@ extern "C" int sb200_moe_align_block_size(const void* topk_ids, int ids_itype, i
   }
   int* scr = (int*)scratch;
   const int ctas = (p.nseg + 7) / 8;
-  moe_align_count_kernel<<<ctas, 256, 0, s>>>(topk_ids, ids_itype, numel, E, p.seg_len, p.nseg, scr,
+  launch_dependent(moe_align_count_kernel, ctas, 256, 0, s, topk_ids, ids_itype, numel, E, p.seg_len, p.nseg, scr,
                                               sorted_token_ids, sorted_capacity);
   SB_CHECK_LAUNCH("moe_align_count_kernel");
-  moe_align_scan_kernel<<<1, 1024, 0, s>>>(E, block_size, p.nseg, scr, expert_ids, expert_ids_capacity,
+  launch_dependent(moe_align_scan_kernel, 1, 1024, 0, s, E, block_size, p.nseg, scr, expert_ids, expert_ids_capacity,
                                            num_tokens_post_pad);
   SB_CHECK_LAUNCH("moe_align_scan_kernel");
-  moe_align_scatter_kernel<<<ctas, 256, 0, s>>>(topk_ids, ids_itype, numel, E, p.seg_len, p.nseg, scr,
+  launch_dependent(moe_align_scatter_kernel, ctas, 256, 0, s, topk_ids, ids_itype, numel, E, p.seg_len, p.nseg, scr,
                                                 sorted_token_ids);
   SB_CHECK_LAUNCH("moe_align_scatter_kernel");
   return SB200_OK;
@@ -520,13 +526,13 @@ extern "C" int sb200_moe_align_block_size_noalloc(const void* topk_ids, int ids_
     return SB200_ERR_UNSUPPORTED;
   }
   const int ctas = (p.nseg + 7) / 8;
-  moe_align_count_kernel<<<ctas, 256, 0, s>>>(topk_ids, ids_itype, numel, E, p.seg_len, p.nseg, scr, sorted_token_ids,
+  launch_dependent(moe_align_count_kernel, ctas, 256, 0, s, topk_ids, ids_itype, numel, E, p.seg_len, p.nseg, scr, sorted_token_ids,
                                               sorted_capacity);
   SB_CHECK_LAUNCH("moe_align_count_kernel (noalloc)");
-  moe_align_scan_kernel<<<1, 1024, 0, s>>>(E, block_size, p.nseg, scr, expert_ids, expert_ids_capacity,
+  launch_dependent(moe_align_scan_kernel, 1, 1024, 0, s, E, block_size, p.nseg, scr, expert_ids, expert_ids_capacity,
                                            num_tokens_post_pad);
   SB_CHECK_LAUNCH("moe_align_scan_kernel (noalloc)");
-  moe_align_scatter_kernel<<<ctas, 256, 0, s>>>(topk_ids, ids_itype, numel, E, p.seg_len, p.nseg, scr,
+  launch_dependent(moe_align_scatter_kernel, ctas, 256, 0, s, topk_ids, ids_itype, numel, E, p.seg_len, p.nseg, scr,
                                                 sorted_token_ids);
   SB_CHECK_LAUNCH("moe_align_scatter_kernel (noalloc)");
   return SB200_OK;

@@ -10,12 +10,15 @@
 
 namespace sb200 {
 
-constexpr int kNormMaxVec = 4;  // 16-byte vectors cached per thread
+constexpr int kNormMaxVec = 4;  // most 16-byte vectors cached per thread
 
-template <typename T, bool ADD, bool VEC>
+// VEC: 16-byte vectors a thread holds (registers decide how many rows an SM works on: 1 whenever a row has at most 512
+// of them), or 0 for the generic path.
+template <typename T, bool ADD, int VEC>
 __global__ void __launch_bounds__(1024)
 rms_norm_kernel(T* __restrict__ out, T* resid_out, const T* x, const T* resid,
                 const T* __restrict__ w, float eps, int H) {
+  grid_dependency_begin();
   __shared__ float red[33];
   constexpr int N = Vec16<T>::N;
   const int64_t row = blockIdx.x;
@@ -25,14 +28,15 @@ rms_norm_kernel(T* __restrict__ out, T* resid_out, const T* x, const T* resid,
   T* zrow = ADD ? resid_out + row * H : nullptr;
   float ss = 0.f;
 
-  if constexpr (VEC) {
-    Vec16<T> cache[kNormMaxVec];
+  if constexpr (VEC > 0) {
+    Vec16<T> cache[VEC], wv[VEC];
     const int nvec = H / N;
 #pragma unroll
-    for (int i = 0; i < kNormMaxVec; ++i) {
+    for (int i = 0; i < VEC; ++i) {
       const int v = i * blockDim.x + threadIdx.x;
       if (v < nvec) {
         cache[i] = ld16(xr + v * N);
+        wv[i] = ld16(w + v * N);  // (needed after the reduction: its latency hides behind that of the row)
         if constexpr (ADD) {
           Vec16<T> r = ld16(rr + v * N);
 #pragma unroll
@@ -47,16 +51,16 @@ rms_norm_kernel(T* __restrict__ out, T* resid_out, const T* x, const T* resid,
         }
       }
     }
-    ss = block_sum(ss, red);
+    ss = block_sum_once(ss, red);
     const float inv = rsqrtf(ss / (float)H + eps);
 #pragma unroll
-    for (int i = 0; i < kNormMaxVec; ++i) {
+    for (int i = 0; i < VEC; ++i) {
       const int v = i * blockDim.x + threadIdx.x;
       if (v < nvec) {
-        Vec16<T> wv = ld16(w + v * N), o;
+        Vec16<T> o;
 #pragma unroll
         for (int j = 0; j < N; ++j)
-          o.v[j] = DT<T>::from_f(rt<T>(DT<T>::to_f(cache[i].v[j]) * inv) * DT<T>::to_f(wv.v[j]));
+          o.v[j] = DT<T>::from_f(rt<T>(DT<T>::to_f(cache[i].v[j]) * inv) * DT<T>::to_f(wv[i].v[j]));
         st16(orow + v * N, o);
       }
     }
@@ -84,25 +88,22 @@ static int launch_norm(void* out, void* resid_out, const void* x, const void* re
   constexpr int N = Vec16<T>::N;
   bool vec = (H % N == 0) && aligned16(out) && aligned16(x) && aligned16(w) &&
              (!ADD || (aligned16(resid) && aligned16(resid_out)));
-  int threads = 0;
+  int threads = 0, per = 1;
   if (vec) {
     const int64_t nvec = H / N;
     // fewest vectors per thread that keep the CTA at >= 128 threads when possible
-    int per = 1;
-    while (per < kNormMaxVec && (nvec + per - 1) / per > 512) ++per;
+    while (per < kNormMaxVec && (nvec + per - 1) / per > 512) per *= 2;
     int64_t t = (nvec + per - 1) / per;
     t = (t + 31) / 32 * 32;
-    if (t > 1024 || t * kNormMaxVec < nvec) vec = false;
+    if (t > 1024) vec = false;
     threads = (int)t;
   }
   if (!vec) threads = (int)((H < 1024 ? (H + 31) / 32 * 32 : 1024));
-  dim3 grid((unsigned)T_);
-  if (vec)
-    rms_norm_kernel<T, ADD, true><<<grid, threads, 0, s>>>((T*)out, (T*)resid_out, (const T*)x,
-                                                           (const T*)resid, (const T*)w, eps, (int)H);
-  else
-    rms_norm_kernel<T, ADD, false><<<grid, threads, 0, s>>>((T*)out, (T*)resid_out, (const T*)x,
-                                                            (const T*)resid, (const T*)w, eps, (int)H);
+  const dim3 grid((unsigned)T_);
+  auto kern = !vec ? rms_norm_kernel<T, ADD, 0> : per == 1 ? rms_norm_kernel<T, ADD, 1>
+              : per == 2 ? rms_norm_kernel<T, ADD, 2> : rms_norm_kernel<T, ADD, kNormMaxVec>;
+  launch_dependent(kern, grid, dim3((unsigned)threads), 0, s, (T*)out, (T*)resid_out, (const T*)x, (const T*)resid, (const T*)w,
+                   eps, (int)H);
   SB_CHECK_LAUNCH("rms_norm_kernel");
   return SB200_OK;
 }

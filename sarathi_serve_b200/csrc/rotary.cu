@@ -20,6 +20,7 @@ template <typename T, bool NEOX, bool VEC>
 __global__ void __launch_bounds__(256)
 rotary_kernel(const int64_t* __restrict__ positions, T* q, T* k, const T* __restrict__ cache,
               int64_t T_, int nq, int nkv, int head_size, int rot_dim, int64_t q_stride, int64_t k_stride) {
+  grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int half = rot_dim / 2;
   const int heads = nq + nkv;
@@ -86,7 +87,7 @@ static int launch_rotary(const int64_t* positions, void* q, void* k, const void*
   if (blocks > cap) blocks = cap;
   T* kq = (T*)q; T* kk = (T*)k; const T* kc = (const T*)cache;
 #define SB_ROT(NE, VE) \
-  rotary_kernel<T, NE, VE><<<(int)blocks, 256, 0, s>>>(positions, kq, kk, kc, T_, nq, nkv, head_size, rot_dim, qs, ks)
+  launch_dependent(rotary_kernel<T, NE, VE>, (int)blocks, 256, 0, s, positions, kq, kk, kc, T_, nq, nkv, head_size, rot_dim, qs, ks)
   if (neox) { if (vec) SB_ROT(true, true); else SB_ROT(true, false); }
   else      { if (vec) SB_ROT(false, true); else SB_ROT(false, false); }
 #undef SB_ROT

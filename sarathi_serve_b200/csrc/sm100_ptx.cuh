@@ -19,6 +19,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // to run on a single lane, so the instructions that take their operands from uniform registers -- TMA, tcgen05.mma,
 // tcgen05.commit -- are issued directly; under a plain lane test the compiler has to assume several active lanes and
 // wraps every one of them in a loop over the lanes, which cost the MMA and TMA threads about 550 clocks per k-block.
+// The TMA and MMA warps run their loops and waits with all lanes and elect only around the issue of a k-block: the
+// warp stays converged for the warp-wide instructions around and after the loops.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
@@ -72,6 +74,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
   }
   return true;
+}
+
+// The same wait made by all lanes of a warp; the result is the same for all of them.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag) ? 1 : 0) != 0;
+  __syncwarp();
+  return ok;
 }
 
 // ----------------------------------------------------------------------- TMA

@@ -210,6 +210,26 @@ def test_linear_silu_mul(dtype, tile_n, T, d, K):
     assert rel_err(out, ref) <= 2e-2
 
 
+def _bf_bound(ref64, absum, K, dtype):
+    """One rounding of the result to the 16-bit type plus K + 64 fp32 roundings of products and sums."""
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    return u * ref64.abs() + (K + 64) * 2.0 ** -24 * absum + 1e-7
+
+
+# The last, partial 128-row block of A is loaded by a shorter box, blocks without rows not at all.
+@pytest.mark.parametrize("tile_n", [128, 2064, 3128, 4064, 203064, 301128, 205064])
+@pytest.mark.parametrize("T", [1, 8, 127, 129, 255, 257, 385])
+def test_linear_partial_row_blocks(tile_n, T):
+    from sarathi_serve_b200 import dense_ops
+    K, N = 512, 192
+    _skip_unless_planned(0, T, N, K, tile_n)
+    x, w = _rand((T, K), torch.bfloat16, T).cuda(), _rand((N, K), torch.bfloat16, 9, 0.05).cuda()
+    out = dense_ops.linear(x, w, tile_n=tile_n)
+    _check_status()
+    ref, absum = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert bool(((out.double() - ref).abs() <= _bf_bound(ref, absum, K, torch.bfloat16)).all())
+
+
 def test_gemm_linearity_full_size():
     """Size-independent property at the headline shapes: (a*x) W^T == a * (x W^T) for a power of two."""
     from sarathi_serve_b200 import dense_ops
