@@ -419,6 +419,11 @@ extern "C" int sb200_gemm_colpar(void* out, int64_t ldo, const void* x, int64_t 
     SB_CHECK_ARG(N % 2 == 0, "gemm_colpar: silu_and_mul epilogue needs an even N");
     epi = EPI_SILU_MUL;
   }
+  if (tile_cfg == 0) {
+    bool done = false;
+    const int rc = run_gemm_narrow(dtype, epi, x, ldx, w, ldw, g, s, &done);
+    if (rc || done) return rc;
+  }
   CommView cv = {};
   ReduceArgs ra = {};
   const GemmPlan plan = plan_gemm(epi, T, N, K, g.head_size, tile_cfg, workspace ? (size_t)workspace_bytes : 0,

@@ -25,6 +25,9 @@ uint32_t gemm_push_increments(const GemmPlan& p, int64_t M, int64_t lo, int64_t 
 int run_gemm_sm100(int dtype, int epi, const GemmPlan& plan, const void* x, int64_t ldx, const void* w, int64_t ldw,
                    GemmArgs g, void* workspace, const CommView& cv, const ReduceArgs& ra, cudaStream_t s,
                    int64_t b_rows = 0);  // b_rows: rows of the B matrix when it is taller than g.N (stacked experts)
+// At most 16 output columns (gemm_narrow.cu); `*done` = false: the problem is not one of that kernel's, nothing was launched.
+int run_gemm_narrow(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g,
+                    cudaStream_t s, bool* done);
 int run_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, const float* B, int64_t ldb, const float* bias,
                  int M, int N, int K, cudaStream_t s);
 

@@ -1,0 +1,91 @@
+// Projections with at most 16 output columns (the router gate of a mixture-of-experts block): out[t, n] = x[t, :] . w[n, :].
+//
+// Bound: latency, then one read of x (8 MB for 1024 tokens of 4096: about 1.3 us).  A tensor-core tile would be mostly
+// padding and its few CTAs would walk all of K one k-block after the other, so this is a dot-product kernel: a CTA takes
+// ROWS tokens and all columns, its eight warps cut K into interleaved slices of 256 elements, a lane keeps
+// ROWS x 8 fp32 sums of its 16-byte pieces (every loaded weight is used for ROWS tokens, every loaded activation for
+// eight columns), and the sums meet in registers and shared memory in a fixed order.
+#include "gemm_host.cuh"
+
+namespace sb200 {
+
+constexpr int kNarrowMaxCols = 16, kNarrowWarps = 8;
+
+template <typename T, int ROWS>
+__global__ void __launch_bounds__(kNarrowWarps * 32)
+gemm_narrow_kernel(const T* __restrict__ x, int64_t ldx, const T* __restrict__ w, int64_t ldw, const GemmArgs g) {
+  __shared__ float part[kNarrowWarps][ROWS * 8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t0 = blockIdx.x * ROWS, n0 = blockIdx.y * 8;
+  grid_dependency_begin();
+  float acc[ROWS][8];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+    for (int n = 0; n < 8; ++n) acc[r][n] = 0.f;
+  for (int k = (warp * 32 + lane) * 8; k < g.K; k += kNarrowWarps * 256) {  // (K is a multiple of 8)
+    Vec16<T> xv[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      xv[r].raw = make_uint4(0, 0, 0, 0);
+      if (t0 + r < g.M) xv[r] = ld16(x + (int64_t)(t0 + r) * ldx + k);
+    }
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      Vec16<T> wv;
+      wv.raw = make_uint4(0, 0, 0, 0);
+      if (n0 + n < g.N) wv = ld16(w + (int64_t)(n0 + n) * ldw + k);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float wf = DT<T>::to_f(wv.v[j]);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[r][n] = fmaf(DT<T>::to_f(xv[r].v[j]), wf, acc[r][n]);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      const float s = warp_sum(acc[r][n]);
+      if (lane == 0) part[warp][r * 8 + n] = s;
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ROWS * 8; i += kNarrowWarps * 32) {
+    const int t = t0 + i / 8, n = n0 + i % 8;
+    if (t >= g.M || n >= g.N) continue;
+    float a = 0.f;
+#pragma unroll
+    for (int v = 0; v < kNarrowWarps; ++v) a += part[v][i];
+    if (g.bias) a += DT<T>::to_f(reinterpret_cast<const T*>(g.bias)[n]);
+    if (g.residual) a = DT<T>::to_f(reinterpret_cast<const T*>(g.residual)[(int64_t)t * g.ldr + n]) + rt<T>(a);
+    reinterpret_cast<T*>(g.out)[(int64_t)t * g.ldo + n] = DT<T>::from_f(a);
+  }
+}
+
+template <typename T>
+static cudaError_t launch_narrow(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g, cudaStream_t s) {
+  const unsigned groups = (unsigned)((g.N + 7) / 8);
+  // eight tokens per CTA reuse the weights most; two while that still leaves SMs without a CTA
+  if (g.M <= 2 * sm_count())
+    return launch_dependent(gemm_narrow_kernel<T, 2>, dim3((unsigned)((g.M + 1) / 2), groups), dim3(kNarrowWarps * 32), 0, s,
+                            (const T*)x, ldx, (const T*)w, ldw, g);
+  return launch_dependent(gemm_narrow_kernel<T, 8>, dim3((unsigned)((g.M + 7) / 8), groups), dim3(kNarrowWarps * 32), 0, s,
+                          (const T*)x, ldx, (const T*)w, ldw, g);
+}
+
+// Rows that the 16-byte loads can read; anything else is left to the tensor-core kernel, which also words the errors.
+static bool narrow_fits(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g) {
+  return epi == EPI_STORE && (dtype == SB200_BF16 || dtype == SB200_F16) && g.N <= kNarrowMaxCols && g.K % 8 == 0 &&
+         ldx >= g.K && ldw >= g.K && ldx % 8 == 0 && ldw % 8 == 0 && aligned16(x) && aligned16(w);
+}
+
+int run_gemm_narrow(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g,
+                    cudaStream_t s, bool* done) {
+  *done = narrow_fits(dtype, epi, x, ldx, w, ldw, g);
+  if (!*done) return SB200_OK;
+  SB_CUDA(dtype == SB200_BF16 ? launch_narrow<__nv_bfloat16>(x, ldx, w, ldw, g, s) : launch_narrow<__half>(x, ldx, w, ldw, g, s));
+  return SB200_OK;
+}
+
+}  // namespace sb200

@@ -216,6 +216,19 @@ def _bf_bound(ref64, absum, K, dtype):
     return u * ref64.abs() + (K + 64) * 2.0 ** -24 * absum + 1e-7
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,N,K", [(1, 1, 8), (3, 8, 4096), (297, 8, 264), (1024, 8, 4096), (24, 16, 2048), (300, 9, 2056)])
+def test_linear_few_columns(dtype, T, N, K):
+    from sarathi_serve_b200 import dense_ops
+    x, w = _rand((T, K + 8), dtype, T + N + K).cuda()[:, 8:], _rand((N, K), dtype, 7 * N + K, 0.05).cuda()
+    b, r = _rand((N,), dtype, 3).cuda(), _rand((T, N), dtype, 4).cuda()
+    out = dense_ops.linear(x, w)
+    ref, absum = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert bool(((out.double() - ref).abs() <= _bf_bound(ref, absum, K, dtype)).all())
+    got = dense_ops.linear(x, w, b, residual=r)
+    assert rel_err(got.float(), r.double() + (ref + b.double()).to(dtype).double()) <= GEMM_TOL[dtype]
+
+
 # The last, partial 128-row block of A is loaded by a shorter box, blocks without rows not at all.
 @pytest.mark.parametrize("tile_n", [128, 2064, 3128, 4064, 203064, 301128, 205064])
 @pytest.mark.parametrize("T", [1, 8, 127, 129, 255, 257, 385])
