@@ -113,6 +113,21 @@ def test_moe_align_block_size(itype, T, k, E, block, scratch):
         assert torch.equal(re_[:npp // block], e[:npp // block])
 
 
+# One slot more than a single CTA takes, segments that end inside a warp's step, one expert, more experts than threads a
+# CTA of the cluster scans at once, and all slots in the last expert.
+@pytest.mark.parametrize("T,k,E,block", [(1024, 1, 8, 64), (1025, 1, 1, 16), (2049, 1, 200, 16), (8192, 6, 128, 128), (1500, 3, 1100, 7)])
+@pytest.mark.parametrize("skew", [False, True])
+def test_align_over_a_cluster(T, k, E, block, skew):
+    g = torch.Generator().manual_seed(T)
+    ids = torch.randint(0, E, (T, k), generator=g).to(torch.int32)
+    if skew:
+        ids.fill_(E - 1)
+    s, e, n = _align(ids.cuda(), E, block, False)
+    os_, oe, on = O.moe_align_block_size(ids.to(torch.int64), block, E)
+    npp = int(on)
+    assert int(n) == npp and torch.equal(s.cpu(), os_) and torch.equal(e[:npp // block].cpu(), oe[:npp // block])
+
+
 def test_align_empty():
     ids = torch.empty(0, 2, dtype=torch.int32, device="cuda")
     s, e, n = _align(ids, 8, 64)
