@@ -139,8 +139,14 @@ def itype_id(t: torch.Tensor) -> int:
         raise RuntimeError(f"unsupported integer dtype {t.dtype}") from None
 
 
+# Handle of the current stream without building a torch.cuda.Stream around it (0.3 us instead of 3.2 us, once per launch).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def require_cuda(*tensors: torch.Tensor) -> None:
