@@ -167,8 +167,8 @@ typedef struct sb200_rotary_args {
 /* out[T, N] = x[T, K] * w[N, K]^T: the local matmul of a ColumnParallelLinear /
  * ReplicatedLinear shard (w is the nn.Linear weight [out_features/tp, in_features],
  * row-major, used as is).  ldx / ldw / ldo are row strides in elements.
- * bf16 / fp16 run on tcgen05 tensor cores with fp32 accumulation; fp32 runs a plain
- * FFMA kernel and supports SB200_EPI_NONE only.
+ * bf16 / fp16 run on tcgen05 tensor cores with fp32 accumulation; fp32 runs on the FMA
+ * pipes and supports SB200_EPI_NONE only.
  *   SB200_EPI_ROTARY   : additionally applies rotary_embedding to the q / k heads
  *                        (out is the fused qkv buffer [T, N]).
  *   SB200_EPI_SILU_MUL : w holds the gate shard in rows [0, N/2) and the up shard in
@@ -188,7 +188,10 @@ typedef struct sb200_rotary_args {
  *   that split its k-blocks and combine their fp32 accumulators through distributed shared memory --
  *   accepted when the problem has at most #SMs / (2 S) tiles and at least S k-blocks (with the
  *   row-parallel epilogue of sb200_gemm_rowpar: S = 2 only, and only as many clusters as the
- *   device reports co-resident, because that kernel's CTAs wait for one another).
+ *   device reports co-resident, because that kernel's CTAs wait for one another); MODE = 6|7: operand
+ *   roles swapped, 128 weight rows times two | one accumulators against BN = 16..256 tokens per
+ *   tile, S = 1..8 CTAs of a cluster share a tile's K (plain, rotary and SiLU epilogues; MODE 7 plain only;
+ *   a rotary layout it does not take is run as tile_cfg 0).
  * workspace: optional device buffer (zero-filled once by the caller, at least 64 KiB +
  *   room for the fp32 partial tiles) that allows tiles to be cut along K;
  *   the library leaves its first 64 KiB zero again after every launch.  NULL / 0: whole

@@ -93,6 +93,31 @@ static int max_coresident_clusters(int cluster_ctas) {
   return n;
 }
 
+// Clocks of one launch, fitted to the kernel's times (most within 15 %), to set against the estimate of gemm_swap.cu; among
+// its own plans plan_gemm's model below chooses better.  The tensor pipe (pairs reach about 5/6 of it), the
+// L2's delivery to shared memory, the issue of a k-block; launch and prologue; the epilogue of the last tile; and for
+// tiles cut along K the trip of their parts through the workspace.
+double gemm_plan_clocks(int epi, int64_t N, int64_t K, const GemmPlan& p) {
+  if (!p.bn) return 1e30;
+  const int busy = p.units * (p.cta2 ? 2 : 1);
+  const double stage = gemm_stage_bytes(p.mi, p.bn, p.cta2), feed = gemm_feed_rate(busy);
+  double per_kb = 2.0 * p.mi * (p.bn > 92 ? p.bn : 92) * (p.cta2 ? 1.2 : 1.0);
+  if (stage / feed > per_kb) per_kb = stage / feed;
+  if (per_kb < 260.0) per_kb = 260.0;
+  const double finish = 1500.0 + (p.mi == 2 ? p.bn / 32.0 : p.bn / 64.0) * (epi == EPI_STORE ? 900.0 : 1300.0);
+  const bool dbuf = p.mi * p.bn * 2 <= 512;
+  const int rem = p.m_tiles * p.n_tiles - p.tiles_full;
+  const double main = p.k_blocks * per_kb, rounds = p.units ? (double)(p.tiles_full / p.units) : 0.0;
+  double c = 6500.0 + rounds * (dbuf ? (main > finish ? main : finish) : main + finish);
+  if (rem == 0) c += dbuf ? finish : 0.0;
+  else if (p.rem_units > rem) c += (double)(((int64_t)rem * p.k_blocks + p.rem_units - 1) / p.rem_units) * per_kb + 8000.0 + 50.0 * p.bn +
+                                   (epi == EPI_ROTARY ? 12000.0 : epi == EPI_SILU_MUL ? 6000.0 : 0.0);
+  else c += main + finish;
+  if (epi == EPI_SILU_MUL) c *= 1.1;
+  const double hbm = (double)N * K * 2 / 3500.0 + 8000.0;
+  return c > hbm ? c : hbm;
+}
+
 // ------------------------------------------------------------ tile selection
 // Analytical choice of (CTA pairing, MI, BN, scheduling): estimated SM clocks of the slowest unit.
 //   main loop per k-block = max(tensor time, shared-memory traffic of the stage at 128 B/clk
@@ -419,15 +444,27 @@ extern "C" int sb200_gemm_colpar(void* out, int64_t ldo, const void* x, int64_t 
     SB_CHECK_ARG(N % 2 == 0, "gemm_colpar: silu_and_mul epilogue needs an even N");
     epi = EPI_SILU_MUL;
   }
+  const int neox = epi == EPI_ROTARY ? g.is_neox : 1, mode = (tile_cfg / 1000) % 100;
+  bool done = false;
   if (tile_cfg == 0) {
-    bool done = false;
     const int rc = run_gemm_narrow(dtype, epi, x, ldx, w, ldw, g, s, &done);
     if (rc || done) return rc;
   }
+  if (tile_cfg == 0 || mode == 6 || mode == 7) {
+    // Up to 64 tokens always (8 tokens x 28672 x 4096: 42 us against 66, 64 tokens: 43 against 56); beyond that where the
+    // estimate is a tenth better: ragged batches (300 tokens x 28672 x 4096: 78 us against 100) and few tiles
+    // (512 x 768 x 4096: 15.5 against 22), while whole 256-row tiles of CTA pairs need half of the operand traffic
+    // (512 tokens x 28672 x 4096: 97 us there, 115 here).
+    double other = 1e30;
+    if (T > 64 && tile_cfg == 0) other = 0.92 * gemm_plan_clocks(epi, N, K, plan_gemm(epi, T, N, K, g.head_size, 0,
+                                                                                   workspace ? (size_t)workspace_bytes : 0, neox));
+    const int rc = run_gemm_swap(dtype, epi, x, ldx, w, ldw, g, neox, tile_cfg, other, s, &done);
+    if (rc || done) return rc;
+    if (mode == 6 || mode == 7) tile_cfg = 0;  // not one of its problems (a head layout it does not take): choose
+  }
   CommView cv = {};
   ReduceArgs ra = {};
-  const GemmPlan plan = plan_gemm(epi, T, N, K, g.head_size, tile_cfg, workspace ? (size_t)workspace_bytes : 0,
-                                  epi == EPI_ROTARY ? g.is_neox : 1);
+  const GemmPlan plan = plan_gemm(epi, T, N, K, g.head_size, tile_cfg, workspace ? (size_t)workspace_bytes : 0, neox);
   return run_gemm_sm100(dtype, epi, plan, x, ldx, w, ldw, g, workspace, cv, ra, s);
 }
 

@@ -25,7 +25,19 @@ uint32_t gemm_push_increments(const GemmPlan& p, int64_t M, int64_t lo, int64_t 
 int run_gemm_sm100(int dtype, int epi, const GemmPlan& plan, const void* x, int64_t ldx, const void* w, int64_t ldw,
                    GemmArgs g, void* workspace, const CommView& cv, const ReduceArgs& ra, cudaStream_t s,
                    int64_t b_rows = 0);  // b_rows: rows of the B matrix when it is taller than g.N (stacked experts)
-// At most 16 output columns (gemm_narrow.cu); `*done` = false: the problem is not one of that kernel's, nothing was launched.
+// Operand roles swapped, tokens as the MMA's N (gemm_swap.cu).
+constexpr int kSwapHalfRing = 104 * 1024;             // ring of one CTA: two of them fit an SM
+constexpr int kSwapRing = 216 * 1024;
+constexpr int64_t kSwapPrefetchBytes = 24ll << 20;    // weights of a launch requested before its dependency wait
+// Clocks a gemm_sm100.cuh launch of this plan takes, fitted like the estimate of gemm_swap.cu it is compared with.
+double gemm_plan_clocks(int epi, int64_t N, int64_t K, const GemmPlan& p);
+// Bytes a clock that the L2 delivers to the shared memory of one SM while `ctas` SMs load.
+inline double gemm_feed_rate(int ctas) { return 8600.0 / ctas < 90.0 ? 8600.0 / ctas : 90.0; }
+// tile_cfg 0: taken when its best plan is estimated below `other_clocks`.  `*done` = false: the problem was left to
+// the caller, nothing was launched.
+int run_gemm_swap(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g, int neox,
+                  int tile_cfg, double other_clocks, cudaStream_t s, bool* done);
+// At most 16 output columns (gemm_narrow.cu); `*done` as above.
 int run_gemm_narrow(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g,
                     cudaStream_t s, bool* done);
 int run_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, const float* B, int64_t ldb, const float* bias,

@@ -742,9 +742,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
         const int p_kb1 = kb_hi(sg);
         for (int kb = kb_lo(sg); kb < p_kb1; ++kb) {
-          if (!ptx::mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+          ok = ptx::mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag) && ok;
           if (kb == kb_lo(sg) && it == 0 && lane == 0) SB_GEMM_MARK(11);  // stage 0 free, about to request it
-          if (ptx::elect_one()) {
+          if (ptx::elect_one() && ok) {
             uint8_t* sa = stage_base + (size_t)stage * stage_bytes;
             uint8_t* sb = sa + a_bytes;
             const bool halves = (EPI == EPI_SILU_MUL) || (EPI == EPI_ROTARY && g.rot_split);  // B tile = two row blocks
@@ -791,10 +791,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               }
             }
           }
-          __syncwarp();
           if (kb == kb_lo(sg) && it == 0 && lane == 0) SB_GEMM_MARK(2);  // first stage requested
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
+        ok = __all_sync(0xffffffffu, ok ? 1 : 0) != 0;
       }
       if (lane == 0) SB_GEMM_MARK(3);  // last stage requested
     }
@@ -816,10 +816,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * MI * BN);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!ptx::mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+          ok = ptx::mbar_wait(&full_bar[stage], phase, abort_flag) && ok;
           ptx::tc_fence_after();
           if (kb == kb0 && it == 0 && lane == 0) SB_GEMM_MARK(4);  // first stage arrived
-          if (ptx::elect_one()) {
+          if (ptx::elect_one() && ok) {
             const uint32_t sa = ptx::smem_u32(stage_base + (size_t)stage * stage_bytes);
             const uint64_t db = ptx::make_smem_desc_sw128(sa + a_bytes);
 #pragma unroll
@@ -836,9 +836,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
             if (CTA2) ptx::umma_commit_pair_mask(&empty_bar[stage], pair_mask); else ptx::umma_commit(&empty_bar[stage]);
           }
-          __syncwarp();
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
+        ok = __all_sync(0xffffffffu, ok ? 1 : 0) != 0;
         if (ok && ptx::elect_one()) {  // accumulators complete (the same lane: a commit covers what its thread issued)
           if (CTA2) ptx::umma_commit_pair_mask(&tmem_full[buf], pair_mask); else ptx::umma_commit(&tmem_full[buf]);
         }

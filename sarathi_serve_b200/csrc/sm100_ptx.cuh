@@ -20,7 +20,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // tcgen05.commit -- are issued directly; under a plain lane test the compiler has to assume several active lanes and
 // wraps every one of them in a loop over the lanes, which cost the MMA and TMA threads about 550 clocks per k-block.
 // The TMA and MMA warps run their loops and waits with all lanes and elect only around the issue of a k-block: the
-// warp stays converged for the warp-wide instructions around and after the loops.
+// warp-wide election brings the lanes together in every step.  (What an MMA warp does between two k-blocks is hardly
+// hidden -- the tensor pipe takes few instructions ahead -- so nothing but the wait and the election stands there.)
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
@@ -93,6 +94,17 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
+      : "memory");
+}
+
+// The same load for data that is read once: its lines are the first to leave the L2, so that a stream of weights does not
+// push out what was requested ahead for the next kernel (or the activations).
+__device__ __forceinline__ void tma_load_2d_once(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1) {
+  uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "l"(policy)
       : "memory");
 }
 

@@ -1,7 +1,7 @@
 """Tensor-level wrappers of the dense projection entry points of the C ABI
 (``sb200_gemm_colpar``): the local matmul of a column-parallel / replicated
 linear layer, optionally with the rotary embedding or SiLU*mul applied in the
-GEMM epilogue.  bf16/fp16 run on tcgen05 tensor cores, fp32 on an FFMA kernel."""
+GEMM epilogue.  bf16/fp16 run on tcgen05 tensor cores, fp32 on the FMA pipes."""
 from __future__ import annotations
 
 import ctypes
@@ -73,7 +73,7 @@ def raise_if_flagged(device: torch.device) -> None:
 
 
 def _ws(x: torch.Tensor):
-    """(pointer, bytes) of the split-K workspace for x's device; fp32 runs the FFMA kernel and needs none."""
+    """(pointer, bytes) of the split-K workspace for x's device; the fp32 kernel needs none."""
     if x.dtype == torch.float32:
         return None, 0
     w = workspace(x.device)
@@ -240,6 +240,11 @@ def _candidates(kind: str, T: int, Nn: int, K: int, head_size: int):
                     continue
                 mode_eff = (2 + p["accumulators"]) if p["cta_pairs"] else p["accumulators"]
                 out.append(p["bn"] + 1000 * mode_eff + 100000 * p["k_parts"])
+    if kind != "push":  # operand roles swapped: tokens per tile in steps of 16, one or two accumulators, K over 1..8 CTAs
+        for tiles in range(-(-T // 256), min(-(-T // 16), -(-T // 256) + 12) + 1):
+            nt = -(-(-(-T // tiles)) // 16) * 16
+            for mode in ((6, 7) if kind == "store" else (6,)):
+                out += [nt + 1000 * mode + 100000 * s for s in (1, 2, 3, 4, 6, 8)]
     return sorted(set(out))
 
 

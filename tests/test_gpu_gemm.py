@@ -210,10 +210,73 @@ def test_linear_silu_mul(dtype, tile_n, T, d, K):
     assert rel_err(out, ref) <= 2e-2
 
 
+# Small batches run on a kernel of their own (tokens as the N side of the MMA, K cut over a cluster): edges of its token
+# granules (8, 16, 64), of its 128-column tiles, of a head's halves, one and many k-blocks, and more tiles than SMs.
 def _bf_bound(ref64, absum, K, dtype):
     """One rounding of the result to the 16-bit type plus K + 64 fp32 roundings of products and sums."""
     u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     return u * ref64.abs() + (K + 64) * 2.0 ** -24 * absum + 1e-7
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,N,K", [(1, 128, 64), (8, 4096, 512), (9, 200, 264), (16, 384, 1000), (17, 17, 4096), (63, 768, 4096),
+                                   (64, 130, 1792), (5, 20000, 128), (64, 19072, 64), (65, 256, 512)])
+def test_linear_small_batch(dtype, T, N, K):
+    from sarathi_serve_b200 import dense_ops
+    x, w = _rand((T, K + 64), dtype, T + N + K).cuda()[:, 64:], _rand((N, K), dtype, 7 * N + K, 0.05).cuda()
+    b, r = _rand((N,), dtype, 3).cuda(), _rand((T, N + 3), dtype, 4).cuda()[:, 3:]
+    out = torch.full((T, N + 1), 7.0, dtype=dtype, device="cuda")
+    dense_ops.linear(x, w, out=out[:, 1:])
+    _check_status()
+    ref, absum = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert bool(((out[:, 1:].double() - ref).abs() <= _bf_bound(ref, absum, K, dtype)).all())
+    assert bool((out[:, 0] == 7.0).all())
+    # bias and residual: the same sums through the other kernel, rounded at the same places
+    got = dense_ops.linear(x, w, b, residual=r)
+    want = dense_ops.linear(x, w, b, residual=r, tile_n=128)
+    assert rel_err(got.float(), want.float()) <= GEMM_TOL[dtype]
+    assert rel_err(got.float(), r.double() + (ref + b.double()).to(dtype).double()) <= GEMM_TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,d,K", [(1, 64, 64), (8, 14336, 256), (16, 96, 520), (31, 1792, 4096), (64, 200, 512)])
+def test_linear_silu_mul_small_batch(dtype, T, d, K):
+    from sarathi_serve_b200 import dense_ops
+    x, w = _rand((T, K), dtype, T + K), _rand((2 * d, K), dtype, d, 0.05)
+    out = dense_ops.linear_silu_mul(x.cuda(), w.cuda())
+    _check_status()
+    ref = O.silu_and_mul((x.float().cuda() @ w.float().cuda().t()).to(dtype).cpu())
+    assert rel_err(out, ref) <= 2e-2
+    assert rel_err(out, dense_ops.linear_silu_mul(x.cuda(), w.cuda(), tile_n=128)) <= 2e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,nq,nkv,hd,K", [(1, 1, 1, 64, 64), (8, 4, 1, 128, 4096), (17, 3, 1, 256, 264), (64, 5, 2, 64, 1024),
+                                           (61, 32, 8, 128, 512)])
+def test_linear_rotary_small_batch(dtype, T, nq, nkv, hd, K):
+    """Against the general kernel (its tiles hold whole heads), with the append to the paged cache."""
+    from sarathi_serve_b200 import dense_ops
+    N, page = (nq + 2 * nkv) * hd, 16
+    x, w = _rand((T, K), dtype, T + K).cuda(), _rand((N, K), dtype, N, 0.03).cuda()
+    g = torch.Generator().manual_seed(5)
+    pos = torch.randint(0, 2048, (T,), generator=g).cuda()
+    cs = O.cos_sin_cache(hd, hd, 2048, 10000.0, dtype).cuda()
+    res = []
+    for cfg in (0, 256):
+        cache = torch.zeros((T + page - 1) // page + 1, 2, page, nkv, hd, dtype=dtype, device="cuda")
+        # distinct slots only: tokens that share one would race
+        s = torch.full((T,), -1, dtype=torch.int64, device="cuda")
+        live = torch.arange(T, device="cuda") % 5 != 0
+        s[live] = (torch.arange(T, device="cuda") // page * 2 * page + torch.arange(T, device="cuda") % page)[live]
+        out = dense_ops.linear_rotary(x, w, pos, cs, hd, (nq + nkv) * hd, True, tile_n=cfg, kv_cache=cache, kv_slots=s,
+                                      num_kv_heads=nkv)
+        _check_status()
+        res.append((out, cache))
+        k, v = out[:, nq * hd:(nq + nkv) * hd], out[:, (nq + nkv) * hd:]
+        flat = cache.view(-1, nkv * hd)
+        assert torch.equal(flat[s[live]], k[live]) and torch.equal(flat[s[live] + page], v[live])
+        assert int((flat.abs().sum(1) > 0).sum()) == 2 * int(live.sum())
+    assert rel_err(res[0][0], res[1][0]) <= GEMM_TOL[dtype]
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -227,6 +290,42 @@ def test_linear_few_columns(dtype, T, N, K):
     assert bool(((out.double() - ref).abs() <= _bf_bound(ref, absum, K, dtype)).all())
     got = dense_ops.linear(x, w, b, residual=r)
     assert rel_err(got.float(), r.double() + (ref + b.double()).to(dtype).double()) <= GEMM_TOL[dtype]
+
+
+# The same kernel on larger, ragged batches: token tiles of 16..256, one and two accumulators, K over a cluster, several
+# rounds of tiles per CTA with one and with two sets of accumulators.
+@pytest.mark.parametrize("cfg", [6016, 6112, 6128, 6256, 7064, 7256, 206064, 807032, 306176])
+@pytest.mark.parametrize("T,N,K", [(65, 256, 512), (129, 200, 1000), (300, 1000, 512), (513, 4096, 576)])
+def test_linear_swapped_tiles(cfg, T, N, K):
+    from sarathi_serve_b200 import dense_ops
+    x, w = _rand((T, K), torch.bfloat16, T + N).cuda(), _rand((N, K), torch.bfloat16, N + K, 0.05).cuda()
+    b, r = _rand((N,), torch.bfloat16, 3).cuda(), _rand((T, N), torch.bfloat16, 4).cuda()
+    out = dense_ops.linear(x, w, tile_n=cfg)
+    _check_status()
+    ref, absum = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert bool(((out.double() - ref).abs() <= _bf_bound(ref, absum, K, torch.bfloat16)).all())
+    got = dense_ops.linear(x, w, b, tile_n=cfg, residual=r)
+    assert rel_err(got.float(), r.double() + (ref + b.double()).to(torch.bfloat16).double()) <= GEMM_TOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("cfg", [6048, 6112, 6256, 206096])
+@pytest.mark.parametrize("T,nq,nkv,hd", [(100, 2, 1, 64), (300, 4, 2, 128), (131, 1, 1, 256)])
+def test_linear_rotary_and_silu_swapped_tiles(cfg, T, nq, nkv, hd):
+    from sarathi_serve_b200 import dense_ops
+    N, K = (nq + 2 * nkv) * hd, 320
+    x, w = _rand((T, K), torch.float16, T).cuda(), _rand((N, K), torch.float16, N, 0.05).cuda()
+    pos = torch.randint(0, 2048, (T,), generator=torch.Generator().manual_seed(5)).cuda()
+    cs = O.cos_sin_cache(hd, hd, 2048, 10000.0, torch.float16).cuda()
+    caches = [torch.zeros(T, 2, 1, nkv, hd, dtype=torch.float16, device="cuda") for _ in range(2)]
+    slots = torch.arange(T, device="cuda").flip(0) * 2
+    outs = [dense_ops.linear_rotary(x, w, pos, cs, hd, (nq + nkv) * hd, True, tile_n=c, kv_cache=kc, kv_slots=slots,
+                                    num_kv_heads=nkv) for c, kc in zip((cfg, 256), caches)]
+    _check_status()
+    assert rel_err(outs[0], outs[1]) <= GEMM_TOL[torch.float16] and rel_err(caches[0], caches[1]) <= GEMM_TOL[torch.float16]
+    assert torch.equal(caches[0].view(T, 2, -1)[slots // 2, 1], outs[0][:, (nq + nkv) * hd:])
+    acts = [dense_ops.linear_silu_mul(x, w, tile_n=c) for c in (cfg, 128)]
+    _check_status()
+    assert rel_err(acts[0], acts[1]) <= 2e-2
 
 
 # The last, partial 128-row block of A is loaded by a shorter box, blocks without rows not at all.
