@@ -452,11 +452,11 @@ extern "C" int sb200_gemm_colpar(void* out, int64_t ldo, const void* x, int64_t 
   }
   if (tile_cfg == 0 || mode == 6 || mode == 7) {
     // Up to 64 tokens always (8 tokens x 28672 x 4096: 42 us against 66, 64 tokens: 43 against 56); beyond that where the
-    // estimate is a tenth better: ragged batches (300 tokens x 28672 x 4096: 78 us against 100) and few tiles
+    // estimate is an eighth better: ragged batches (300 tokens x 28672 x 4096: 78 us against 100) and few tiles
     // (512 x 768 x 4096: 15.5 against 22), while whole 256-row tiles of CTA pairs need half of the operand traffic
     // (512 tokens x 28672 x 4096: 97 us there, 115 here).
     double other = 1e30;
-    if (T > 64 && tile_cfg == 0) other = 0.92 * gemm_plan_clocks(epi, N, K, plan_gemm(epi, T, N, K, g.head_size, 0,
+    if (T > 64 && tile_cfg == 0) other = 0.87 * gemm_plan_clocks(epi, N, K, plan_gemm(epi, T, N, K, g.head_size, 0,
                                                                                    workspace ? (size_t)workspace_bytes : 0, neox));
     const int rc = run_gemm_swap(dtype, epi, x, ldx, w, ldw, g, neox, tile_cfg, other, s, &done);
     if (rc || done) return rc;

@@ -20,6 +20,8 @@
 //     next projection's CTAs are resident while this one drains, and before they wait for its results they ask for
 //     their first weights -- into the L2 only, where a late write to the weights by an earlier kernel is still seen.
 //     EW = 8 and the whole SM otherwise.
+#include <atomic>
+
 #include "gemm_host.cuh"
 
 namespace sb200 {
@@ -366,6 +368,39 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 }
 
 // ------------------------------------------------------------------- planning
+// Clusters of `split` CTAs that run at once, as the runtime reports them.  A cluster has to fit inside one GPC, so these
+// are fewer CTAs than there are SMs, and the tiles beyond them wait for a second round that costs as much as the first
+// (18 clusters of eight, 24 of six: qkv of a TP=8 rank, 512 tokens, took 30 us against 21 in the general kernel).
+static int swap_clusters(int split, int ew) {
+  static std::atomic<int> cache[16][2][9];  // [device][ew][split]; 0 = not asked yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16 || split < 1 || split > 8) return sm_count() / (split < 1 ? 1 : split);
+  std::atomic<int>& c = cache[dev][ew == 4 ? 0 : 1][split];
+  int n = c.load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  // (the dynamic shared memory decides; the other epilogues' kernels differ in registers only)
+  const void* kern = ew == 4 ? (const void*)gemm_swap_kernel<__nv_bfloat16, EPI_STORE, 1, 4> : (const void*)gemm_swap_kernel<__nv_bfloat16, EPI_STORE, 1, 8>;
+  const int smem = (ew == 4 ? kSwapHalfRing : kSwapRing) + 2048;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(sm_count() / split * split));
+  cfg.blockDim = dim3((unsigned)(64 + 32 * ew));
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    n = 1;  // not answered: no tile is cut
+  }
+  c.store(n, std::memory_order_relaxed);
+  return n;
+}
+
 // A plan for `nacc` accumulators, t_tiles token tiles and `split` CTAs per tile; false when it does not fit.
 static bool swap_plan(int epi, int64_t M, int64_t N, int64_t K, int head_size, int nacc, int t_tiles, int split, SwapPlan* p) {
   const int sms = sm_count();
@@ -412,14 +447,16 @@ static double swap_cost(int epi, int64_t N, int64_t K, const SwapPlan& p) {
   if (p.nacc == 2 && feed > 60.0) feed = 60.0;                     // three to five boxes a stage
   if (stage / feed > per_kb) per_kb = stage / feed;
   if (per_kb < 430.0) per_kb = 430.0;                              // issue
+  if (epi == EPI_ROTARY) per_kb += 1.5 * p.nt;                     // measured: 16 k-blocks of 160 tokens 27 us, 64 of 176 52
   if (p.stages <= 3) per_kb *= 1.2;                                // too shallow to hide a load
   const double chunks = p.nt / 16, warps = p.ew / 4;
   const double finish = 600.0 + chunks / warps * (epi == EPI_SILU_MUL ? 900.0 : epi == EPI_ROTARY ? 3000.0 : 350.0 * p.nacc);
   const int64_t tiles = (int64_t)p.w_tiles * p.t_tiles;
   double c = 6000.0;
   if (p.split > 1) {  // cluster launch, two cluster barriers, the exchange
-    const int64_t rounds = (tiles * p.split + sms - 1) / sms;
-    c += (double)rounds * ((p.k_blocks + p.split - 1) / p.split) * per_kb + 8000.0 + p.nt * p.nacc * 30.0 / warps +
+    const int clusters = swap_clusters(p.split, p.ew);
+    const int64_t rounds = (tiles + clusters - 1) / clusters;
+    c += (double)rounds * ((p.k_blocks + p.split - 1) / p.split) * per_kb + 8000.0 + p.nt * p.nacc * (epi == EPI_ROTARY ? 60.0 : 30.0) / warps +
          (epi == EPI_ROTARY ? 3000.0 : 0.0) + finish / p.split;
   } else {
     const int64_t rounds = (tiles + p.grid - 1) / p.grid;
@@ -457,6 +494,7 @@ static bool search_swap(int epi, int64_t M, int64_t N, int64_t K, int head_size,
         SwapPlan p;
         if (!swap_plan(epi, M, N, K, head_size, nacc, (int)t, s, &p)) continue;
         if (s > 1 && ((int64_t)p.w_tiles * t * s > sm_count() || p.k_blocks / s < 4)) break;
+        if (s > 1 && (int64_t)p.w_tiles * t > swap_clusters(s, p.ew)) continue;  // one round of clusters
         const double c = swap_cost(epi, N, K, p);
         if (c < *cost) { *cost = c; *best = p; }
       }
