@@ -328,6 +328,23 @@ def test_linear_rotary_and_silu_swapped_tiles(cfg, T, nq, nkv, hd):
     assert rel_err(acts[0], acts[1]) <= 2e-2
 
 
+# The library's own choice on both sides of its rule: K cut over clusters that all run at once, whole tiles, CTA pairs.
+@pytest.mark.parametrize("T", [33, 65, 130, 270, 513])
+@pytest.mark.parametrize("nq,nkv", [(4, 1), (8, 2), (16, 4)])
+def test_linear_rotary_and_silu_chosen_tiles(T, nq, nkv):
+    from sarathi_serve_b200 import dense_ops
+    hd, K = 128, 2048
+    N = (nq + 2 * nkv) * hd
+    x, w = _rand((T, K), torch.float16, T).cuda(), _rand((N, K), torch.float16, N, 0.05).cuda()
+    pos = torch.randint(0, 2048, (T,), generator=torch.Generator().manual_seed(6)).cuda()
+    cs = O.cos_sin_cache(hd, hd, 2048, 10000.0, torch.float16).cuda()
+    outs = [dense_ops.linear_rotary(x, w, pos, cs, hd, (nq + nkv) * hd, True, tile_n=c) for c in (0, 128)]
+    acts = [dense_ops.linear_silu_mul(x, w, tile_n=c) for c in (0, 128)]
+    _check_status()
+    assert rel_err(outs[0], outs[1]) <= GEMM_TOL[torch.float16]
+    assert rel_err(acts[0], acts[1]) <= 2e-2
+
+
 # The last, partial 128-row block of A is loaded by a shorter box, blocks without rows not at all.
 @pytest.mark.parametrize("tile_n", [128, 2064, 3128, 4064, 203064, 301128, 205064])
 @pytest.mark.parametrize("T", [1, 8, 127, 129, 255, 257, 385])
