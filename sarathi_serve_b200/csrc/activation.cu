@@ -30,7 +30,7 @@ template <typename T> __device__ __forceinline__ float gelu_fast_op(float x) {
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
-silu_and_mul_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t T_, int64_t d) {
+silu_and_mul_kernel(T* out, const T* in, int64_t T_, int64_t d) {
   grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -75,7 +75,7 @@ silu_and_mul_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t T_, i
 
 template <typename T, int OP, bool VEC>
 __global__ void __launch_bounds__(256)
-unary_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t total) {
+unary_kernel(T* out, const T* in, int64_t total) {
   grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;

@@ -74,6 +74,10 @@ __host__ __device__ inline size_t dtype_size(int dt) { return dt == SB200_F32 ? 
 // `grid_launch_dependents` lets the NEXT kernel of the stream be scheduled as soon as every CTA of this one has
 // executed it and an SM has room: what overlaps is launch latency and prologues.  A kernel that owns TMEM executes it
 // after its allocation, so that no CTA of a later kernel can hold the TMEM an earlier one still needs.
+// What such a kernel reads may be written while it is already running, until its wait returns.  So its pointers are not
+// `__restrict__` and it never loads through the read-only path (`__ldg`, ld.global.nc): both tell the compiler that the
+// memory does not change during the kernel, and with that it may move the load ahead of the wait.  This holds for
+// weights and norm vectors too: any of them can be the result of the kernel before.
 // (2048 x 28672 x 4096 back to back: 318 -> 312 us; 300 x 4096 x 4096: 25.6 -> 23.6 us.)
 namespace ptx {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

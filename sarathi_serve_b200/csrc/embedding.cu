@@ -11,7 +11,7 @@ namespace sb200 {
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
-vocab_embedding_kernel(T* __restrict__ out, const int64_t* __restrict__ ids, const T* __restrict__ weight, int64_t T_,
+vocab_embedding_kernel(T* out, const int64_t* ids, const T* weight, int64_t T_,
                        int64_t H, int64_t vocab_start, int64_t vocab_end) {
   grid_dependency_begin();
   constexpr int N = Vec16<T>::N;

@@ -33,12 +33,12 @@ __device__ __forceinline__ float2 f32x2_split(unsigned long long v) {
 
 // Four consecutive k of one row (zeros outside the matrix).  VEC: rows are 16-byte aligned and K is a multiple of 4.
 template <bool VEC>
-__device__ __forceinline__ float4 f32_load4(const float* __restrict__ p, int64_t ld, int row, int rows, int k, int K) {
+__device__ __forceinline__ float4 f32_load4(const float* p, int64_t ld, int row, int rows, int k, int K) {
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   if (row < rows && k < K) {
     const float* q = p + (int64_t)row * ld + k;
     if (VEC) {
-      v = __ldg(reinterpret_cast<const float4*>(q));
+      v = *reinterpret_cast<const float4*>(q);
     } else {
       v.x = q[0];
       if (k + 1 < K) v.y = q[1];
@@ -50,7 +50,7 @@ __device__ __forceinline__ float4 f32_load4(const float* __restrict__ p, int64_t
 }
 
 // Four consecutive output columns of one row.
-__device__ __forceinline__ void f32_store4(float* __restrict__ C, int64_t ldc, const float* __restrict__ bias, int m, int n,
+__device__ __forceinline__ void f32_store4(float* C, int64_t ldc, const float* bias, int m, int n,
                                            int M, int N, float4 v, bool vec) {
   if (m >= M || n >= N) return;
   float* c = C + (int64_t)m * ldc + n;
@@ -70,8 +70,8 @@ __device__ __forceinline__ void f32_store4(float* __restrict__ C, int64_t ldc, c
 // Warps: 2 x 2 over the BM x 128 tile; in a warp, lane = 8 * ty + tx covers rows ty*4 (+ 16) and columns tx*4 (+ 32).
 template <int BM, bool VEC>
 __global__ void __launch_bounds__(kF32Threads, 3)
-gemm_f32_kernel(float* __restrict__ C, int64_t ldc, const float* __restrict__ A, int64_t lda,
-                const float* __restrict__ B, int64_t ldb, const float* __restrict__ bias, int M, int N, int K, int vec_c) {
+gemm_f32_kernel(float* C, int64_t ldc, const float* A, int64_t lda,
+                const float* B, int64_t ldb, const float* bias, int M, int N, int K, int vec_c) {
   constexpr int TM = BM / 8, LDA = BM + 4, LDB = kF32BN + 4;  // (+4: the transposing stores conflict two ways at most)
   constexpr int A_LD = BM / 32, B_LD = kF32BN / 32;           // 16-byte loads per thread and k-tile
   constexpr int kTile = kF32BK * (LDA + LDB);

@@ -13,7 +13,7 @@ constexpr int kNarrowMaxCols = 16, kNarrowWarps = 8;
 
 template <typename T, int ROWS>
 __global__ void __launch_bounds__(kNarrowWarps * 32)
-gemm_narrow_kernel(const T* __restrict__ x, int64_t ldx, const T* __restrict__ w, int64_t ldw, const GemmArgs g) {
+gemm_narrow_kernel(const T* x, int64_t ldx, const T* w, int64_t ldw, const GemmArgs g) {
   __shared__ float part[kNarrowWarps][ROWS * 8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t0 = blockIdx.x * ROWS, n0 = blockIdx.y * 8;

@@ -20,9 +20,9 @@ namespace sb200 {
 // slots[i] = page * (2 * page_size) + slot: the row of cache seen as [pages * 2 * page_size, kv_heads * head_dim]
 // that receives token i's key; its value goes page_size rows further.  -1 for entries with a negative
 // batch index (padding tokens).
-__global__ void kv_slots_kernel(int64_t* __restrict__ slots, const int32_t* __restrict__ batch_indices,
-                                const int32_t* __restrict__ positions, const int32_t* __restrict__ kv_indices,
-                                const int32_t* __restrict__ kv_indptr, int64_t n, int page_size) {
+__global__ void kv_slots_kernel(int64_t* slots, const int32_t* batch_indices,
+                                const int32_t* positions, const int32_t* kv_indices,
+                                const int32_t* kv_indptr, int64_t n, int page_size) {
   grid_dependency_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -35,8 +35,8 @@ __global__ void kv_slots_kernel(int64_t* __restrict__ slots, const int32_t* __re
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-kv_append_kernel(T* __restrict__ cache, const T* __restrict__ k, int64_t ldk, const T* __restrict__ v, int64_t ldv,
-                 const int64_t* __restrict__ slots, int64_t n, int row_elems, int page_size) {
+kv_append_kernel(T* cache, const T* k, int64_t ldk, const T* v, int64_t ldv,
+                 const int64_t* slots, int64_t n, int row_elems, int page_size) {
   grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int nvec = row_elems / N;

@@ -15,8 +15,8 @@ constexpr int kMoeBlockRows = 128;
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-moe_gather_kernel(T* __restrict__ out, const T* __restrict__ x, const int32_t* __restrict__ sorted_ids,
-                  const int32_t* __restrict__ num_post_pad, int64_t rows_cap, int64_t num_slots, int H, int top_k) {
+moe_gather_kernel(T* out, const T* x, const int32_t* sorted_ids,
+                  const int32_t* num_post_pad, int64_t rows_cap, int64_t num_slots, int H, int top_k) {
   grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int nvec = H / N;
@@ -36,7 +36,7 @@ moe_gather_kernel(T* __restrict__ out, const T* __restrict__ x, const int32_t* _
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-moe_sum_kernel(T* __restrict__ out, const T* __restrict__ in3, const T* __restrict__ residual, int64_t T_, int k, int H) {
+moe_sum_kernel(T* out, const T* in3, const T* residual, int64_t T_, int k, int H) {
   grid_dependency_begin();
   constexpr int N = Vec16<T>::N;
   const int nvec = H / N;

@@ -40,8 +40,8 @@ template <int E> struct TopkLayout {
 
 template <int E, typename TIn, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
-topk_softmax_pow2_kernel(const TIn* __restrict__ gating, float* __restrict__ weights, int32_t* __restrict__ ids,
-                         int32_t* __restrict__ src_rows, int64_t num_rows, int k, int renorm) {
+topk_softmax_pow2_kernel(const TIn* gating, float* weights, int32_t* ids,
+                         int32_t* src_rows, int64_t num_rows, int k, int renorm) {
   grid_dependency_begin();
   using L = TopkLayout<E>;
   constexpr int VPT = L::VPT, TPR = L::TPR, EPL = L::ELTS_PER_LDG, LDGS = L::VECS;
@@ -116,8 +116,8 @@ topk_softmax_pow2_kernel(const TIn* __restrict__ gating, float* __restrict__ wei
 // as in moeSoftmax (csrc/moe_topk_softmax_kernels.cu:50-106).
 template <typename TIn>
 __global__ void __launch_bounds__(256)
-topk_softmax_generic_kernel(const TIn* __restrict__ gating, float* __restrict__ weights, int32_t* __restrict__ ids,
-                            int32_t* __restrict__ src_rows, int64_t num_rows, int E, int k, int renorm) {
+topk_softmax_generic_kernel(const TIn* gating, float* weights, int32_t* ids,
+                            int32_t* src_rows, int64_t num_rows, int E, int k, int renorm) {
   grid_dependency_begin();
   constexpr int TPB = 256;
   using BlockReduce = cub::BlockReduce<float, TPB>;

@@ -16,8 +16,8 @@ constexpr int kNormMaxVec = 4;  // most 16-byte vectors cached per thread
 // of them), or 0 for the generic path.
 template <typename T, bool ADD, int VEC>
 __global__ void __launch_bounds__(1024)
-rms_norm_kernel(T* __restrict__ out, T* resid_out, const T* x, const T* resid,
-                const T* __restrict__ w, float eps, int H) {
+rms_norm_kernel(T* out, T* resid_out, const T* x, const T* resid,
+                const T* w, float eps, int H) {
   grid_dependency_begin();
   __shared__ float red[33];
   constexpr int N = Vec16<T>::N;

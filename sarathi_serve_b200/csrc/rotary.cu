@@ -18,7 +18,7 @@ __device__ __forceinline__ void rot_pair(float x, float y, float c, float s, flo
 
 template <typename T, bool NEOX, bool VEC>
 __global__ void __launch_bounds__(256)
-rotary_kernel(const int64_t* __restrict__ positions, T* q, T* k, const T* __restrict__ cache,
+rotary_kernel(const int64_t* positions, T* q, T* k, const T* cache,
               int64_t T_, int nq, int nkv, int head_size, int rot_dim, int64_t q_stride, int64_t k_stride) {
   grid_dependency_begin();
   constexpr int N = Vec16<T>::N;

@@ -199,3 +199,69 @@ def test_vocab_parallel_embedding_module_tp1():
         assert out.shape == (5, 13, 256) and torch.equal(out.cpu(), w[ids])
     finally:
         ps.destroy_model_parallel()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T", [3, 600])  # (600: block alignment over a cluster)
+def test_chain_of_small_kernels_on_shared_buffers(dtype, T):
+    """Kernels start while their predecessor still runs: a chain in which every kernel reads what the one before has just
+    written, over buffers that are written again and again, gives the same bits as with the device idle between any two."""
+    from sarathi_serve_b200 import (activation_ops, dense_ops, embedding_ops, kv_cache_ops, layernorm_ops, moe_ops,
+                                    pos_encoding_ops)
+    H, E, page, heads, hd = 512, 8, 16, 8, 64
+    g = torch.Generator().manual_seed(T)
+
+    def rand(*shape, scale=1.0):
+        return (torch.randn(*shape, generator=g) * scale).to(dtype).cuda()
+    start, w, wide, gate, cs = rand(T, H), rand(H), rand(2 * H, H, scale=0.05), rand(E, H, scale=0.05), rand(64, hd)
+    table, pos = rand(64, H), torch.randint(0, 64, (T,), generator=g).cuda()
+    a, b, c = (torch.empty(T, H, dtype=dtype, device="cuda") for _ in range(3))
+    two = torch.empty(T, 2 * H, dtype=dtype, device="cuda")
+    logits = torch.empty(T, E, dtype=dtype, device="cuda")
+    tw, ids = torch.empty(T, 2, device="cuda"), torch.empty(T, 2, dtype=torch.int32, device="cuda")
+    rows = T * 2 + E * 15
+    srt, eid, npp = (torch.empty(n, dtype=torch.int32, device="cuda") for n in (rows, (rows + 15) // 16, 1))
+    cache = torch.zeros((T + page - 1) // page, 2, page, heads, hd, dtype=dtype, device="cuda")
+    slots = (torch.arange(T) // page * 2 * page + torch.arange(T) % page).cuda()
+    zero = torch.zeros(T, dtype=torch.int32, device="cuda")
+    positions = torch.arange(T, dtype=torch.int32, device="cuda")
+    indices = torch.arange(cache.shape[0], dtype=torch.int32, device="cuda")
+    indptr = torch.tensor([0, cache.shape[0]], dtype=torch.int32, device="cuda")
+    steps = [lambda: layernorm_ops.rms_norm(b, a, w, 1e-5),
+             lambda: dense_ops.linear(b, wide, out=two),
+             lambda: activation_ops.silu_and_mul(b, two),
+             lambda: layernorm_ops.fused_add_rms_norm(c, a, b, a, w, 1e-5),
+             lambda: dense_ops.linear(c, gate, out=logits),
+             lambda: moe_ops.topk_softmax(tw, ids, None, logits, renormalize=True),
+             lambda: moe_ops.moe_align_block_size(ids, E, 16, srt, eid, npp),
+             lambda: embedding_ops.vocab_embedding(b, pos, table, 0, 64),
+             lambda: pos_encoding_ops.rotary_embedding(pos, b, c, hd, cs, True),
+             lambda: kv_cache_ops.slots(zero, positions, indices, indptr, page, out=slots),
+             lambda: kv_cache_ops.append_rows(cache, c.view(T, heads, hd), b.view(T, heads, hd), slots),
+             lambda: activation_ops.gelu_new(a, c)]
+    seen = [a, b, c, two, logits, tw, ids, srt, npp, cache]
+
+    def chain(wait):
+        for _ in range(3):
+            for s in steps:
+                s()
+                if wait:
+                    torch.cuda.synchronize()
+    a.copy_(start)
+    chain(True)
+    want = [t.clone() for t in seen]
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        chain(False)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        a.copy_(start)
+        chain(False)
+    for i in range(50):
+        for t in seen[1:-1]:
+            t.fill_(i % 7)
+        cache.zero_()  # (rows no token owns keep what they hold)
+        graph.replay()
+        assert all(torch.equal(x, y) for x, y in zip(seen, want)), i

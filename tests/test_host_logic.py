@@ -497,3 +497,53 @@ def test_prepare_inputs_lays_a_mixed_batch_out_like_the_reference():
     assert pad_to_alignment([], 8) == [] and len(pad_to_alignment([1] * 9, 8)) == 16
     tok, pos, n = prepare_inputs([], [], "cpu")
     assert n == 0 and tok.numel() == 0
+
+
+# ------------------------------------------- kernels that start while their predecessor still writes their inputs
+def _kernel_signatures():
+    """(file, kernel, parameter list, body) of every __global__ function of the library's sources."""
+    import glob
+    import re
+    from sarathi_serve_b200 import build
+    for path in sorted(glob.glob(os.path.join(build.CSRC, "*.cu")) + glob.glob(os.path.join(build.CSRC, "*.cuh"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__", text):
+            head = re.compile(r"(\w+)\(((?:[^()]|\([^()]*\))*)\)\s*\{").search(text, m.end())
+            body = text[head.end():text.find("\n}\n", head.end())]
+            yield os.path.basename(path), head.group(1), head.group(2), body
+
+
+def test_early_started_kernels_make_no_promise_about_their_inputs():
+    """A kernel with a dependency wait runs while the kernel before it still writes what it is going to read.
+    `__restrict__` pointers and read-only loads promise the compiler that this memory does not change, which lets it
+    load ahead of the wait."""
+    import glob
+    from sarathi_serve_b200 import build
+    waiting = [(f, k, params) for f, k, params, body in _kernel_signatures()
+               if "grid_dependency_begin()" in body or "grid_dependency_wait()" in body]
+    names = {k for _, k, _ in waiting}
+    assert {"rms_norm_kernel", "moe_gather_kernel", "gemm_narrow_kernel", "gemm_f32_kernel", "gemm_swap_kernel", "gemm_sm100_kernel",
+            "silu_and_mul_kernel", "kv_append_kernel", "vocab_embedding_kernel", "topk_softmax_pow2_kernel", "rotary_kernel",
+            "moe_align_cluster_kernel"} <= names
+    assert [(f, k) for f, k, params in waiting if "__restrict__" in params] == []
+    files = {f for f, _, _ in waiting}
+    for path in glob.glob(os.path.join(build.CSRC, "*")):
+        text = open(path).read()
+        code = "\n".join(line.split("//")[0] for line in text.splitlines())
+        assert "__ldg" not in code and "ld.global.nc" not in code, path
+        if os.path.basename(path) in files:  # inlined helpers of these kernels
+            assert "__restrict__" not in code, path
+
+
+def test_launches_with_early_start_go_with_a_wait():
+    """Every kernel handed to launch_dependent waits for its predecessor before anything else."""
+    import glob
+    import re
+    from sarathi_serve_b200 import build
+    bodies = {k: body for _, k, _, body in _kernel_signatures()}
+    launched = set()
+    for path in glob.glob(os.path.join(build.CSRC, "*.cu")):
+        launched |= set(re.findall(r"launch_dependent\((\w+_kernel)", open(path).read()))
+    assert len(launched) >= 12
+    for k in launched:
+        assert "grid_dependency_begin()" in bodies[k], k
