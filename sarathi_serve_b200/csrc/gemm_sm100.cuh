@@ -989,7 +989,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         ptx::tc_fence_after();
       }
       ptx::tc_fence_before();
-      __syncthreads();          // (the warps re-converge here: the producer and the MMA issuer ran on one lane)
+      __syncwarp();  // the block barrier and the cluster barrier are warp-wide: every warp arrives as a whole
+      __syncthreads();
       ptx::cluster_sync_all();  // every pair's MMAs are complete: the stage buffers of all CTAs are free
       ptx::tc_fence_after();
       if (warp == 2 && lane == 0) SB_GEMM_MARK(6);

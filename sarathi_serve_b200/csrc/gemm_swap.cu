@@ -46,6 +46,7 @@ struct SwapPlan {
 // 32 lanes x 16 consecutive TMEM columns.
 __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, float* f) {
   uint32_t r[16];
+  __syncwarp();  // .aligned
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
       "tcgen05.wait::ld.sync.aligned;"

@@ -547,3 +547,18 @@ def test_launches_with_early_start_go_with_a_wait():
     assert len(launched) >= 12
     for k in launched:
         assert "grid_dependency_begin()" in bodies[k], k
+
+
+def test_warp_wide_instructions_join_the_warp_first():
+    """An `.aligned` instruction executed by part of a warp is undefined: each one in the sources follows a __syncwarp."""
+    import glob
+    from sarathi_serve_b200 import build
+    found = 0
+    for path in sorted(glob.glob(os.path.join(build.CSRC, "*.cu*"))):
+        lines = [line.split("//")[0] for line in open(path).read().splitlines()]
+        for i, line in enumerate(lines):
+            if ".aligned" not in line or "wait::ld" in line:  # (tcgen05.wait::ld: in one statement with its load)
+                continue
+            found += 1
+            assert any("__syncwarp();" in prev for prev in lines[max(0, i - 4):i]), f"{path}:{i + 1}"
+    assert found >= 11
