@@ -190,8 +190,11 @@ typedef struct sb200_rotary_args {
  *   row-parallel epilogue of sb200_gemm_rowpar: S = 2 only, and only as many clusters as the
  *   device reports co-resident, because that kernel's CTAs wait for one another); MODE = 6|7: operand
  *   roles swapped, 128 weight rows times two | one accumulators against BN = 16..256 tokens per
- *   tile, S = 1..8 CTAs of a cluster share a tile's K (plain, rotary and SiLU epilogues; MODE 7 plain only;
- *   a rotary layout it does not take is run as tile_cfg 0).
+ *   tile, S = 1..8 CTAs of a cluster share a tile's K (plain, rotary and SiLU epilogues; MODE 7 plain only).
+ *   BN is the most tokens of a tile: the tokens are spread evenly over ceil(T / BN) tiles, in steps of 16.
+ *   Refused (SB200_ERR_INVALID_ARGUMENT) where it does not fit: BN < 16 or > 256, S > 8 or more than the
+ *   k-blocks, an exchange larger than the stage ring.  A head layout it does not take (GPT-J style rotary
+ *   embedding) is run as tile_cfg 0.
  * workspace: optional device buffer (zero-filled once by the caller, at least 64 KiB +
  *   room for the fp32 partial tiles) that allows tiles to be cut along K;
  *   the library leaves its first 64 KiB zero again after every launch.  NULL / 0: whole

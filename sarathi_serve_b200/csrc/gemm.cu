@@ -257,6 +257,32 @@ GemmPlan plan_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, int 
   return best;
 }
 
+GemmChoice choose_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, size_t ws_bytes) {
+  GemmChoice c = {};
+  const int mode = (tile_cfg / 1000) % 100;
+  bool swapped_only = mode == 6 || mode == 7;
+  if (swapped_only && epi == EPI_ROTARY && !neox) {  // a tuned configuration does not say which head layout it is for
+    tile_cfg = 0;
+    swapped_only = false;
+  }
+  if (!swapped_only && (tile_cfg != 0 || M > 64 || epi == EPI_PUSH))
+    c.general = plan_gemm(epi, M, N, K, head_size, tile_cfg, ws_bytes, neox);
+  if (epi != EPI_PUSH && (tile_cfg == 0 || swapped_only)) {
+    // Up to 64 tokens always (8 tokens x 28672 x 4096: 42 us against 66, 64 tokens: 43 against 56); beyond that where the
+    // estimate is an eighth better: ragged batches (300 tokens x 28672 x 4096: 78 us against 100) and few tiles
+    // (512 x 768 x 4096: 15.5 against 22), while whole 256-row tiles of CTA pairs need half of the operand traffic
+    // (512 tokens x 28672 x 4096: 97 us there, 115 here).
+    double clocks = 0.0;
+    if (plan_swap(epi, M, N, K, head_size, neox, tile_cfg, &c.swapped, &clocks) &&
+        (swapped_only || M <= 64 || clocks < 0.87 * gemm_plan_clocks(epi, N, K, c.general)))
+      c.kernel = GEMM_SWAPPED;
+    else if (!swapped_only && M <= 64)  // (a head layout the swapped kernel does not take)
+      c.general = plan_gemm(epi, M, N, K, head_size, tile_cfg, ws_bytes, neox);
+  }
+  if (c.kernel == GEMM_NONE && c.general.bn) c.kernel = GEMM_GENERAL;
+  return c;
+}
+
 // Arrivals the row-parallel kernel of a rank counts for the rank that owns
 // rows [lo, hi): one per (tile, epilogue slot whose 32 rows overlap the range), times the number of
 // K-parts for tiles that are cut or split inside a cluster (every part finishes a share of such a tile and
@@ -444,28 +470,19 @@ extern "C" int sb200_gemm_colpar(void* out, int64_t ldo, const void* x, int64_t 
     SB_CHECK_ARG(N % 2 == 0, "gemm_colpar: silu_and_mul epilogue needs an even N");
     epi = EPI_SILU_MUL;
   }
-  const int neox = epi == EPI_ROTARY ? g.is_neox : 1, mode = (tile_cfg / 1000) % 100;
-  bool done = false;
   if (tile_cfg == 0) {
+    bool done = false;
     const int rc = run_gemm_narrow(dtype, epi, x, ldx, w, ldw, g, s, &done);
     if (rc || done) return rc;
   }
-  if (tile_cfg == 0 || mode == 6 || mode == 7) {
-    // Up to 64 tokens always (8 tokens x 28672 x 4096: 42 us against 66, 64 tokens: 43 against 56); beyond that where the
-    // estimate is an eighth better: ragged batches (300 tokens x 28672 x 4096: 78 us against 100) and few tiles
-    // (512 x 768 x 4096: 15.5 against 22), while whole 256-row tiles of CTA pairs need half of the operand traffic
-    // (512 tokens x 28672 x 4096: 97 us there, 115 here).
-    double other = 1e30;
-    if (T > 64 && tile_cfg == 0) other = 0.87 * gemm_plan_clocks(epi, N, K, plan_gemm(epi, T, N, K, g.head_size, 0,
-                                                                                   workspace ? (size_t)workspace_bytes : 0, neox));
-    const int rc = run_gemm_swap(dtype, epi, x, ldx, w, ldw, g, neox, tile_cfg, other, s, &done);
-    if (rc || done) return rc;
-    if (mode == 6 || mode == 7) tile_cfg = 0;  // not one of its problems (a head layout it does not take): choose
-  }
+  const GemmChoice c = choose_gemm(epi, T, N, K, g.head_size, epi == EPI_ROTARY ? g.is_neox : 1, tile_cfg,
+                                   workspace ? (size_t)workspace_bytes : 0);
+  SB_CHECK_ARG(c.kernel != GEMM_NONE, "no GEMM tile shape fits epilogue %d, T=%lld N=%lld K=%lld, head_size=%d, tile_cfg=%d", epi,
+               (long long)T, (long long)N, (long long)K, g.head_size, tile_cfg);
+  if (c.kernel == GEMM_SWAPPED) return run_gemm_swap(dtype, epi, c.swapped, x, ldx, w, ldw, g, s);
   CommView cv = {};
   ReduceArgs ra = {};
-  const GemmPlan plan = plan_gemm(epi, T, N, K, g.head_size, tile_cfg, workspace ? (size_t)workspace_bytes : 0, neox);
-  return run_gemm_sm100(dtype, epi, plan, x, ldx, w, ldw, g, workspace, cv, ra, s);
+  return run_gemm_sm100(dtype, epi, c.general, x, ldx, w, ldw, g, workspace, cv, ra, s);
 }
 
 #ifdef SB200_TRACE

@@ -33,13 +33,36 @@ constexpr int64_t kSwapPrefetchBytes = 24ll << 20;    // weights of a launch req
 double gemm_plan_clocks(int epi, int64_t N, int64_t K, const GemmPlan& p);
 // Bytes a clock that the L2 delivers to the shared memory of one SM while `ctas` SMs load.
 inline double gemm_feed_rate(int ctas) { return 8600.0 / ctas < 90.0 ? 8600.0 / ctas : 90.0; }
-// tile_cfg 0: taken when its best plan is estimated below `other_clocks`.  `*done` = false: the problem was left to
-// the caller, nothing was launched.
-int run_gemm_swap(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g, int neox,
-                  int tile_cfg, double other_clocks, cudaStream_t s, bool* done);
-// At most 16 output columns (gemm_narrow.cu); `*done` as above.
+struct SwapPlan {
+  int w_tiles, t_tiles;  // tiles of 128 * nacc weight rows, and of `nt` tokens
+  int nt;         // tokens of a tile: the MMA's N
+  int split;      // CTAs of the cluster that shares a tile's K (1: whole tiles, walked round-robin)
+  int grid;       // CTAs
+  int stages;
+  int act_rows;   // rows of the x box of a full tile (the last tile may have a shorter one)
+  int prefetch;   // k-blocks of weights requested into the L2 before the dependency wait
+  int tmem_cols;
+  int k_blocks;
+  int half_shift; // EPI_ROTARY: log2(head_size / 2)
+  int nacc, ew;   // accumulators and epilogue warps: which kernel
+};
+// tile_cfg 0: the cheapest plan and its estimated clocks; else the plan of that configuration (MODE 6|7).  False: none.
+bool plan_swap(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, SwapPlan* plan, double* clocks);
+int run_gemm_swap(int dtype, int epi, const SwapPlan& plan, const void* x, int64_t ldx, const void* w, int64_t ldw,
+                  const GemmArgs& g, cudaStream_t s);
+// At most 16 output columns (gemm_narrow.cu).  `fits`: the shape; `*done` = false: the operands' rows cannot be read in 16-byte
+// pieces, nothing was launched.
+bool narrow_fits(int epi, int64_t N, int64_t K);
 int run_gemm_narrow(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g,
                     cudaStream_t s, bool* done);
+// Which tensor-core kernel runs a problem, with its schedule.
+enum { GEMM_NONE = 0, GEMM_GENERAL = 1, GEMM_SWAPPED = 2 };
+struct GemmChoice {
+  int kernel;
+  GemmPlan general;
+  SwapPlan swapped;
+};
+GemmChoice choose_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, size_t ws_bytes);
 int run_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, const float* B, int64_t ldb, const float* bias,
                  int M, int N, int K, cudaStream_t s);
 

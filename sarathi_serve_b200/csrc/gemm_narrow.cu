@@ -74,15 +74,13 @@ static cudaError_t launch_narrow(const void* x, int64_t ldx, const void* w, int6
                           (const T*)x, ldx, (const T*)w, ldw, g);
 }
 
-// Rows that the 16-byte loads can read; anything else is left to the tensor-core kernel, which also words the errors.
-static bool narrow_fits(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g) {
-  return epi == EPI_STORE && (dtype == SB200_BF16 || dtype == SB200_F16) && g.N <= kNarrowMaxCols && g.K % 8 == 0 &&
-         ldx >= g.K && ldw >= g.K && ldx % 8 == 0 && ldw % 8 == 0 && aligned16(x) && aligned16(w);
-}
+bool narrow_fits(int epi, int64_t N, int64_t K) { return epi == EPI_STORE && N <= kNarrowMaxCols && K % 8 == 0; }
 
 int run_gemm_narrow(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g,
                     cudaStream_t s, bool* done) {
-  *done = narrow_fits(dtype, epi, x, ldx, w, ldw, g);
+  // rows that the 16-byte loads can read; anything else is left to the tensor-core kernel, which also words the errors
+  *done = narrow_fits(epi, g.N, g.K) && (dtype == SB200_BF16 || dtype == SB200_F16) && ldx >= g.K && ldw >= g.K &&
+          ldx % 8 == 0 && ldw % 8 == 0 && aligned16(x) && aligned16(w);
   if (!*done) return SB200_OK;
   SB_CUDA(dtype == SB200_BF16 ? launch_narrow<__nv_bfloat16>(x, ldx, w, ldw, g, s) : launch_narrow<__half>(x, ldx, w, ldw, g, s));
   return SB200_OK;

@@ -29,20 +29,6 @@ namespace sb200 {
 constexpr int kSwapStages = 8;
 constexpr int kSwapTileBytes = 128 * kBK * 2;  // one accumulator's weights of a stage
 
-struct SwapPlan {
-  int w_tiles, t_tiles;  // tiles of 128 * NACC weight rows, and of `nt` tokens
-  int nt;         // tokens of a tile: the MMA's N
-  int split;      // CTAs of the cluster that shares a tile's K (1: whole tiles, walked round-robin)
-  int grid;       // CTAs
-  int stages;
-  int act_rows;   // rows of the x box of a full tile (the last tile may have a shorter one)
-  int prefetch;   // k-blocks of weights requested into the L2 before the dependency wait
-  int tmem_cols;
-  int k_blocks;
-  int half_shift; // EPI_ROTARY: log2(head_size / 2)
-  int nacc, ew;   // which kernel
-};
-
 // 32 lanes x 16 consecutive TMEM columns.
 __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, float* f) {
   uint32_t r[16];
@@ -502,20 +488,8 @@ static bool search_swap(int epi, int64_t M, int64_t N, int64_t K, int head_size,
   return *cost < 1e30;
 }
 
-static bool plan_swap(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, SwapPlan* best, double* cost) {
-  if (!swap_fits(epi, M, N, head_size, neox)) return false;
-  // the last plans of this thread (a search looks at some 200 of them, a model asks for the same few over and over)
-  struct Entry { int epi, head_size, tile_cfg, sms; int64_t M, N, K; bool found; SwapPlan plan; double cost; };
-  static thread_local Entry memo[64];
-  Entry& e = memo[(size_t)(M * 31 + N * 7 + K + epi) % 64];
-  const int sms = sm_count();
-  if (e.sms == sms && e.epi == epi && e.head_size == head_size && e.tile_cfg == tile_cfg && e.M == M && e.N == N && e.K == K) {
-    *best = e.plan; *cost = e.cost;
-    return e.found;
-  }
-  const bool found = search_swap(epi, M, N, K, head_size, tile_cfg, best, cost);
-  e = Entry{epi, head_size, tile_cfg, sms, M, N, K, found, *best, *cost};
-  return found;
+bool plan_swap(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, SwapPlan* plan, double* clocks) {
+  return swap_fits(epi, M, N, head_size, neox) && search_swap(epi, M, N, K, head_size, tile_cfg, plan, clocks);
 }
 
 template <typename T, int EPI, int NACC, int EW>
@@ -558,13 +532,12 @@ static int dispatch_swap(int epi, const CUtensorMap& tw, const CUtensorMap& tx, 
 #undef SB_SWAP
 }
 
-int run_gemm_swap(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g, int neox,
-                  int tile_cfg, double other_clocks, cudaStream_t s, bool* done) {
-  SwapPlan p;
-  double cost = 0.0;
-  *done = (dtype == SB200_BF16 || dtype == SB200_F16) && plan_swap(epi, g.M, g.N, g.K, g.head_size, neox, tile_cfg, &p, &cost) &&
-          (tile_cfg > 0 || cost < other_clocks);
-  if (!*done) return SB200_OK;
+int run_gemm_swap(int dtype, int epi, const SwapPlan& p, const void* x, int64_t ldx, const void* w, int64_t ldw,
+                  const GemmArgs& g, cudaStream_t s) {
+  if (dtype != SB200_BF16 && dtype != SB200_F16) {
+    set_error("tcgen05 GEMM supports bf16/fp16 only");
+    return SB200_ERR_UNSUPPORTED;
+  }
   CUtensorMap tw, tx, txt;
   int rc = make_tmap_2d(&tx, dtype, x, g.M, g.K, ldx, p.act_rows, kBK);
   if (rc) return rc;

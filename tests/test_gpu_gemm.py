@@ -328,6 +328,17 @@ def test_linear_rotary_and_silu_swapped_tiles(cfg, T, nq, nkv, hd):
     assert rel_err(acts[0], acts[1]) <= 2e-2
 
 
+# Explicit configurations that do not fit are refused, not run as something else: too few and too many tokens a tile, more
+# parts than k-blocks, more than eight, an exchange larger than the ring, two accumulators' epilogue on one.
+@pytest.mark.parametrize("epi,cfg", [("store", 6008), ("store", 6300), ("store", 806064), ("store", 906064), ("store", 206256),
+                                     ("silu", 7064)])
+def test_swapped_tiles_that_do_not_fit_are_refused(epi, cfg):
+    from sarathi_serve_b200 import dense_ops
+    x, w = _rand((256, 256), torch.bfloat16, 1).cuda(), _rand((512, 256), torch.bfloat16, 2, 0.05).cuda()
+    with pytest.raises(RuntimeError, match="no GEMM tile shape fits"):
+        dense_ops.linear(x, w, tile_n=cfg) if epi == "store" else dense_ops.linear_silu_mul(x, w, tile_n=cfg)
+
+
 # The library's own choice on both sides of its rule: K cut over clusters that all run at once, whole tiles, CTA pairs.
 @pytest.mark.parametrize("T", [33, 65, 130, 270, 513])
 @pytest.mark.parametrize("nq,nkv", [(4, 1), (8, 2), (16, 4)])

@@ -562,3 +562,15 @@ def test_warp_wide_instructions_join_the_warp_first():
             found += 1
             assert any("__syncwarp();" in prev for prev in lines[max(0, i - 4):i]), f"{path}:{i + 1}"
     assert found >= 11
+
+
+# ------------------------------------------------------- planner of the swapped projections (host-only)
+@pytest.mark.skipif(torch.cuda.is_available(), reason="makes calls on addresses that are not device memory")
+@pytest.mark.parametrize("epi,cfg", [(0, 6008), (0, 6300), (0, 806064), (0, 906064), (0, 206256), (2, 7064)])
+def test_explicit_swapped_configurations_that_do_not_fit_are_refused(epi, cfg):
+    """256 x 512 x 256: refused before any CUDA call, like every other tile configuration that does not exist."""
+    from sarathi_serve_b200 import _native as N_
+    lib = N_.lib()
+    assert lib.sb200_gemm_colpar(4096, 512, 4096, 256, 4096, 256, None, None, 0, 256, 512, 256, 2, epi, None, None, cfg, None, 0,
+                                 None) == 1
+    assert b"no GEMM tile shape fits" in lib.sb200_last_error()
