@@ -226,14 +226,24 @@ int sb200_kv_cache_slots(int64_t* slots, const int32_t* batch_indices, const int
 int sb200_kv_cache_append(void* cache, const void* k, int64_t ldk, const void* v, int64_t ldv, const int64_t* slots,
                           int64_t n, int num_kv_heads, int head_dim, int page_size, int dtype, sb200_stream_t stream);
 
-/* The tile shape and schedule the two GEMM entry points would pick (epilogue 3 = the
- * row-parallel kernel): out[0..11] = cta_pairs, accumulators, BN, scheduling units,
- * tiles handed out whole, S of the configuration, units that share the k-blocks of the
- * remaining tiles (= their number when nothing is cut), pipeline stages, M tiles, N tiles,
- * k-blocks, CTA pairs per tile (> 1: MODE 5, the tile's k-blocks are split inside a cluster).
- * Host-only; no counterpart in the reference. */
+/* The tile shape and schedule of the general tensor-core kernel (epilogue 3 = the row-parallel
+ * kernel, which always is that one; sb200_gemm_launch says which kernel a column-parallel call
+ * takes): out[0..11] = cta_pairs, accumulators, BN, scheduling units, tiles handed out whole,
+ * S of the configuration, units that share the k-blocks of the remaining tiles (= their number
+ * when nothing is cut), pipeline stages, M tiles, N tiles, k-blocks, CTA pairs per tile (> 1:
+ * MODE 5, the tile's k-blocks are split inside a cluster).  Host-only; no counterpart in the
+ * reference. */
 int sb200_gemm_plan(int epilogue, int64_t T, int64_t N, int64_t K, int head_size, int tile_cfg,
                     int64_t workspace_bytes, int* out);
+
+/* The launch sb200_gemm_colpar makes of a bf16 / fp16 problem with 16-byte aligned rows, for tuning
+ * and tests.  out[0] = 0: the general kernel, out[1..12] as sb200_gemm_plan; 1: operand roles
+ * swapped, out[1..12] = accumulators, tokens per tile, token tiles, weight tiles, CTAs that share a
+ * tile's K, CTAs, pipeline stages, epilogue warps, TMEM columns, k-blocks, sets of accumulators, rounds
+ * of tiles per CTA; 2: the dot-product kernel of at most 16 columns.  SB200_ERR_UNSUPPORTED: the call
+ * would be refused.  Host-only; no counterpart in the reference. */
+int sb200_gemm_launch(int epilogue, int64_t T, int64_t N, int64_t K, int head_size, int is_neox, int tile_cfg,
+                      int64_t workspace_bytes, int* out);
 
 /* Diagnostic: clocks the tensor pipe takes for `iters` k-blocks of four tcgen05.mma (bf16, K = 16 each) with
  * M = 128 on one CTA (pair = 0) or M = 256 on a CTA pair (pair = 1) and N columns, both operands resident in

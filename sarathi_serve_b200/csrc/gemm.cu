@@ -495,18 +495,54 @@ extern "C" int sb200_debug_gemm_trace(unsigned long long* host_out /*[64][16]*/,
 }
 #endif
 
-// The tile shape and schedule sb200_gemm_colpar / sb200_gemm_rowpar would use (for tuning and tests).
+static int epi_of(int epilogue) {
+  return epilogue == SB200_EPI_ROTARY ? EPI_ROTARY : epilogue == SB200_EPI_SILU_MUL ? EPI_SILU_MUL : epilogue == 3 ? EPI_PUSH : EPI_STORE;
+}
+
+static void write_plan(const GemmPlan& p, int* out) {
+  const int v[12] = {p.cta2, p.mi, p.bn, p.units, p.tiles_full, p.rem_splits, p.rem_units, p.stages, p.m_tiles,
+                     p.n_tiles, p.k_blocks, p.cluster_split > 1 ? p.cluster_split : 1};
+  for (int i = 0; i < 12; ++i) out[i] = v[i];
+}
+
+// The general kernel's tile shape and schedule (sb200_gemm_launch: which kernel a call takes).
 // out[0..11] = cta2, mi, bn, units, tiles_full, rem_splits, rem_units, stages, m_tiles, n_tiles, k_blocks, cluster_split.
 extern "C" int sb200_gemm_plan(int epilogue, int64_t T, int64_t N, int64_t K, int head_size, int tile_cfg,
                                int64_t workspace_bytes, int* out) {
   SB_CHECK_ARG(out != nullptr && T > 0 && N > 0 && K > 0, "gemm_plan: bad arguments");
-  const int epi = epilogue == SB200_EPI_ROTARY ? EPI_ROTARY : epilogue == SB200_EPI_SILU_MUL ? EPI_SILU_MUL
-                  : epilogue == 3 ? EPI_PUSH : EPI_STORE;
-  const GemmPlan p = plan_gemm(epi, T, N, K, head_size ? head_size : 128, tile_cfg, (size_t)workspace_bytes);
-  const int v[12] = {p.cta2, p.mi, p.bn, p.units, p.tiles_full, p.rem_splits, p.rem_units, p.stages, p.m_tiles,
-                     p.n_tiles, p.k_blocks, p.cluster_split > 1 ? p.cluster_split : 1};
-  for (int i = 0; i < 12; ++i) out[i] = v[i];
+  const GemmPlan p = plan_gemm(epi_of(epilogue), T, N, K, head_size ? head_size : 128, tile_cfg, (size_t)workspace_bytes);
+  write_plan(p, out);
   return p.bn ? SB200_OK : SB200_ERR_UNSUPPORTED;
+}
+
+// The launch sb200_gemm_colpar makes of a bf16 / fp16 problem: out[0] = kernel, then its schedule (see the header).
+extern "C" int sb200_gemm_launch(int epilogue, int64_t T, int64_t N, int64_t K, int head_size, int is_neox, int tile_cfg,
+                                 int64_t workspace_bytes, int* out) {
+  SB_CHECK_ARG(out != nullptr && T > 0 && N > 0 && K > 0 && T <= INT32_MAX && N <= INT32_MAX && K <= INT32_MAX && epilogue >= 0 &&
+                   epilogue <= SB200_EPI_SILU_MUL, "gemm_launch: bad arguments");
+  const int epi = epi_of(epilogue);
+  for (int i = 0; i < 13; ++i) out[i] = 0;
+  if (tile_cfg == 0 && narrow_fits(epi, N, K)) {
+    out[0] = 2;
+    return SB200_OK;
+  }
+  const GemmChoice c = choose_gemm(epi, T, N, K, head_size ? head_size : 128, epi == EPI_ROTARY ? is_neox : 1, tile_cfg,
+                                   (size_t)workspace_bytes);
+  if (c.kernel == GEMM_NONE) {
+    set_error("no GEMM tile shape fits epilogue %d, T=%lld N=%lld K=%lld, head_size=%d, tile_cfg=%d", epi, (long long)T, (long long)N,
+              (long long)K, head_size, tile_cfg);
+    return SB200_ERR_UNSUPPORTED;
+  }
+  if (c.kernel == GEMM_SWAPPED) {
+    const SwapPlan& p = c.swapped;
+    const int64_t tiles = (int64_t)p.w_tiles * p.t_tiles;
+    const int v[13] = {1, p.nacc, p.nt, p.t_tiles, p.w_tiles, p.split, p.grid, p.stages, p.ew, p.tmem_cols, p.k_blocks,
+                       2 * p.nacc * p.nt <= p.tmem_cols ? 2 : 1, p.split > 1 ? 1 : (int)((tiles + p.grid - 1) / p.grid)};
+    for (int i = 0; i < 13; ++i) out[i] = v[i];
+    return SB200_OK;
+  }
+  write_plan(c.general, out + 1);
+  return SB200_OK;
 }
 
 // Arrivals the row-parallel kernel of one rank counts for the owner of rows [lo, hi) under the schedule

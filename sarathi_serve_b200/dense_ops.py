@@ -180,18 +180,35 @@ def linear_silu_mul(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.T
     return out
 
 
+_PLAN_KEYS = ("cta_pairs", "accumulators", "bn", "units", "tiles_full", "k_parts", "rem_units", "stages", "m_tiles",
+              "n_tiles", "k_blocks", "cluster_split")
+_SWAP_KEYS = ("accumulators", "tokens", "token_tiles", "weight_tiles", "k_parts", "ctas", "stages", "epilogue_warps",
+              "tmem_columns", "k_blocks", "accumulator_sets", "rounds")
+
+
 def gemm_plan(epilogue: int, T: int, Nn: int, K: int, head_size: int = 128, tile_cfg: int = 0,
               workspace_bytes: int = WORKSPACE_BYTES) -> dict:
-    """The tile shape / schedule the library would use for a [T, K] x [Nn, K]^T projection."""
+    """The general tensor-core kernel's tile shape / schedule for a [T, K] x [Nn, K]^T projection (epilogue 3: the
+    row-parallel kernel).  ``gemm_launch`` says which kernel a column-parallel call takes."""
     out = (ctypes.c_int * 12)()
     N.check(N.lib().sb200_gemm_plan(epilogue, T, Nn, K, head_size, tile_cfg, workspace_bytes, out), "gemm_plan")
-    keys = ("cta_pairs", "accumulators", "bn", "units", "tiles_full", "k_parts", "rem_units", "stages", "m_tiles",
-            "n_tiles", "k_blocks", "cluster_split")
-    return dict(zip(keys, out))
+    return dict(zip(_PLAN_KEYS, out))
+
+
+def gemm_launch(epilogue: int, T: int, Nn: int, K: int, head_size: int = 128, tile_cfg: int = 0, is_neox: bool = True,
+                workspace_bytes: int = WORKSPACE_BYTES) -> dict:
+    """The launch a bf16 / fp16 projection makes: ``kernel`` = "general" | "swapped" | "narrow" and its schedule;
+    RuntimeError where the call is refused."""
+    out = (ctypes.c_int * 13)()
+    N.check(N.lib().sb200_gemm_launch(epilogue, T, Nn, K, head_size, 1 if is_neox else 0, tile_cfg, workspace_bytes, out),
+            "gemm_launch")
+    kernel = ("general", "swapped", "narrow")[out[0]]
+    return {"kernel": kernel, **dict(zip({"general": _PLAN_KEYS, "swapped": _SWAP_KEYS}.get(kernel, ()), out[1:]))}
 
 
 # ---------------------------------------------------------------- autotuning
 _tuned: dict = {}
+_KIND_EPI = {"store": EPI_NONE, "rotary": EPI_ROTARY, "silu": EPI_SILU_MUL, "push": 3}
 
 
 def save_tuned(path: str) -> None:
@@ -210,7 +227,13 @@ def load_tuned(path: str) -> int:
     with open(path) as fh:
         rows = json.load(fh)
     for r in rows:
-        _tuned[(r["kind"], int(r["T"]), int(r["N"]), int(r["K"]), getattr(torch, r["dtype"]))] = int(r["cfg"])
+        kind, T, Nn, K, cfg = r["kind"], int(r["T"]), int(r["N"]), int(r["K"]), int(r["cfg"])
+        if (cfg // 1000) % 100 in (6, 7):  # files may hold such numbers for shapes that were run as the default
+            try:
+                gemm_launch(_KIND_EPI[kind], T, Nn, K, tile_cfg=cfg)
+            except RuntimeError:
+                cfg = 0
+        _tuned[(kind, T, Nn, K, getattr(torch, r["dtype"]))] = cfg
     return len(rows)
 
 
@@ -220,7 +243,7 @@ def tuned_cfg(kind: str, T: int, Nn: int, K: int, dtype: torch.dtype) -> int:
 
 
 def _candidates(kind: str, T: int, Nn: int, K: int, head_size: int):
-    epi = {"store": EPI_NONE, "rotary": EPI_ROTARY, "silu": EPI_SILU_MUL, "push": 3}[kind]
+    epi = _KIND_EPI[kind]
     seen, out = set(), []
     for mode in (1, 3, 4, 5):
         for bn in (64, 96, 128, 160, 192, 224, 256):
@@ -244,7 +267,15 @@ def _candidates(kind: str, T: int, Nn: int, K: int, head_size: int):
         for tiles in range(-(-T // 256), min(-(-T // 16), -(-T // 256) + 12) + 1):
             nt = -(-(-(-T // tiles)) // 16) * 16
             for mode in ((6, 7) if kind == "store" else (6,)):
-                out += [nt + 1000 * mode + 100000 * s for s in (1, 2, 3, 4, 6, 8)]
+                for s in (1, 2, 3, 4, 6, 8):
+                    cfg = nt + 1000 * mode + 100000 * s
+                    try:
+                        key = tuple(gemm_launch(epi, T, Nn, K, head_size, cfg).values())
+                    except RuntimeError:
+                        continue
+                    if key not in seen:
+                        seen.add(key)
+                        out.append(cfg)
     return sorted(set(out))
 
 

@@ -574,3 +574,82 @@ def test_explicit_swapped_configurations_that_do_not_fit_are_refused(epi, cfg):
     assert lib.sb200_gemm_colpar(4096, 512, 4096, 256, 4096, 256, None, None, 0, 256, 512, 256, 2, epi, None, None, cfg, None, 0,
                                  None) == 1
     assert b"no GEMM tile shape fits" in lib.sb200_last_error()
+
+
+def test_tuned_files_with_configurations_that_do_not_fit(tmp_path):
+    """A file may name such a configuration (the default was run under its number): it is read as the default."""
+    import json
+    from sarathi_serve_b200 import dense_ops as D
+    saved = dict(D._tuned)
+    try:
+        path = tmp_path / "tuned.json"
+        rows = [("store", 256, 512, 256, 206256), ("store", 256, 512, 256 * 64, 206064), ("silu", 256, 512, 256, 7064),
+                ("push", 512, 4096, 2048, 101128)]
+        path.write_text(json.dumps([dict(kind=k, T=t, N=n, K=kk, dtype="bfloat16", cfg=c) for k, t, n, kk, c in rows]))
+        assert D.load_tuned(str(path)) == 4
+        got = [D.tuned_cfg(k, t, n, kk, torch.bfloat16) for k, t, n, kk, _ in rows]
+        assert got == [0, 206064, 0, 101128]
+    finally:
+        D._tuned.clear()
+        D._tuned.update(saved)
+
+
+@pytest.mark.parametrize("T", [1, 8, 17, 64, 65, 300, 513, 777, 1601, 2048])
+@pytest.mark.parametrize("epi,N,K", [(1, 6144, 4096), (0, 4096, 4096), (2, 28672, 4096), (0, 4096, 14336), (1, 768, 4096), (0, 200, 264),
+                                     (0, 128256, 4096), (2, 200, 64), (1, 192, 64)])
+def test_swapped_launches_are_consistent(T, epi, N, K):
+    """sb200_gemm_launch needs no GPU (148 SMs assumed): every launch it reports covers its problem and fits an SM."""
+    from sarathi_serve_b200 import dense_ops as D
+    hd = 64 if N == 192 else 128
+    p = D.gemm_launch(epi, T, N, K, hd)
+    assert p["kernel"] == "swapped" or T > 64
+    if p["kernel"] == "general":
+        q = D.gemm_plan(epi, T, N, K, hd)
+        assert {k: p[k] for k in q} == q
+    for cfg in (0, 6016, 6128, 6256, 7096, 206048, 406112):
+        try:
+            p = D.gemm_launch(epi, T, N, K, hd, cfg)
+        except RuntimeError:
+            assert cfg != 0
+            continue
+        if p["kernel"] != "swapped":
+            assert cfg == 0
+            continue
+        assert p["tokens"] % 16 == 0 and 16 <= p["tokens"] <= (256 if cfg == 0 else cfg % 1000)
+        assert (p["token_tiles"] - 1) * p["tokens"] < T <= p["token_tiles"] * p["tokens"]
+        acc = p["accumulators"]
+        assert acc == (1 if epi == 0 and cfg // 1000 % 100 != 6 else 2)
+        assert (p["weight_tiles"] - 1) * 128 * acc < N <= p["weight_tiles"] * 128 * acc
+        assert p["k_blocks"] == -(-K // 64) and 1 <= p["k_parts"] <= min(8, p["k_blocks"])
+        tiles = p["token_tiles"] * p["weight_tiles"]
+        if p["k_parts"] > 1:
+            assert p["ctas"] == tiles * p["k_parts"] and p["rounds"] == 1 and (cfg or p["ctas"] <= 148)
+        else:
+            assert p["ctas"] == min(tiles, 148) and p["rounds"] == -(-tiles // p["ctas"])
+        rows = -(-T // 8) * 8 if p["token_tiles"] == 1 else p["tokens"]
+        half = p["epilogue_warps"] == 4
+        assert 2 <= p["stages"] <= 8 and p["stages"] * (acc * 16384 + rows * 128) <= (104 if half else 216) * 1024
+        columns = p["tmem_columns"]
+        assert columns in (32, 64, 128, 256, 512) and acc * p["tokens"] * p["accumulator_sets"] <= columns <= (256 if half else 512)
+        if p["k_parts"] > 1:  # the partial sums of the exchange live in the ring
+            assert p["k_parts"] * -(-p["tokens"] // p["k_parts"]) * acc * 512 <= p["stages"] * (acc * 16384 + rows * 128)
+
+
+def test_which_kernel_a_projection_takes():
+    from sarathi_serve_b200 import dense_ops as D
+    assert D.gemm_launch(0, 1024, 8, 4096)["kernel"] == "narrow" and D.gemm_launch(0, 1024, 16, 4096)["kernel"] == "narrow"
+    assert D.gemm_launch(0, 4, 17, 4096)["kernel"] == "swapped"
+    assert D.gemm_launch(0, 4, 8, 4100)["kernel"] == "swapped"                       # rows that are no multiple of 16 bytes
+    assert D.gemm_launch(1, 4, 768, 4096, is_neox=False)["kernel"] == "general"      # pairs of a GPT-J head sit side by side
+    assert D.gemm_launch(1, 300, 768, 4096, is_neox=False, tile_cfg=6064)["kernel"] == "general"
+    assert D.gemm_launch(2, 300, 28672, 4096)["kernel"] == "swapped" and D.gemm_launch(2, 2048, 28672, 4096)["kernel"] == "general"
+    assert D.gemm_launch(0, 8, 4096, 4096, tile_cfg=128)["kernel"] == "general"
+
+
+def test_autotune_candidates_are_distinct_launches():
+    """Every configuration that is timed exists and is another launch than the rest."""
+    from sarathi_serve_b200 import dense_ops as D
+    for kind, epi, T, N, K in (("store", 0, 2048, 4096, 4096), ("silu", 2, 300, 28672, 4096), ("rotary", 1, 61, 6144, 4096)):
+        cfgs = D._candidates(kind, T, N, K, 128)
+        launches = [tuple(D.gemm_launch(epi, T, N, K, 128, c).items()) for c in cfgs]
+        assert len(set(launches)) == len(cfgs) and any(x[0] == ("kernel", "swapped") for x in launches)
