@@ -245,6 +245,10 @@ int sb200_gemm_plan(int epilogue, int64_t T, int64_t N, int64_t K, int head_size
 int sb200_gemm_launch(int epilogue, int64_t T, int64_t N, int64_t K, int head_size, int is_neox, int tile_cfg,
                       int64_t workspace_bytes, int* out);
 
+/* How many times the calling thread has searched for a schedule: calls whose problem it remembers make no
+ * search.  Host-only, for tests; no counterpart in the reference. */
+int64_t sb200_gemm_choices_made(void);
+
 /* Diagnostic: clocks the tensor pipe takes for `iters` k-blocks of four tcgen05.mma (bf16, K = 16 each) with
  * M = 128 on one CTA (pair = 0) or M = 256 on a CTA pair (pair = 1) and N columns, both operands resident in
  * shared memory (no loads in the timed loop).  dev_clocks[0] = SM clocks until the last MMA was issued,

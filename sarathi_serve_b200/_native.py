@@ -50,6 +50,7 @@ _GEMM_SIGS: dict = {
     "sb200_moe_sum_all_reduce": (_I, [_P, _P, _P, _L, _I, _L, _I, _P, _P, _PP]),
     "sb200_gemm_plan": (_I, [_I, _L, _L, _L, _I, _I, _L, ctypes.POINTER(c_int)]),
     "sb200_gemm_launch": (_I, [_I, _L, _L, _L, _I, _I, _I, _L, ctypes.POINTER(c_int)]),
+    "sb200_gemm_choices_made": (_L, []),
     "sb200_kv_cache_slots": (_I, [_P, _P, _P, _P, _P, _L, _I, _P]),
     "sb200_kv_cache_append": (_I, [_P, _P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _P]),
     "sb200_diag_mma_rate": (_I, [_I, _I, _I, _P, _P]),

@@ -257,7 +257,10 @@ GemmPlan plan_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, int 
   return best;
 }
 
-GemmChoice choose_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, size_t ws_bytes) {
+static thread_local int64_t choices_made = 0;
+
+static GemmChoice search_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, size_t ws_bytes) {
+  ++choices_made;
   GemmChoice c = {};
   const int mode = (tile_cfg / 1000) % 100;
   bool swapped_only = mode == 6 || mode == 7;
@@ -281,6 +284,36 @@ GemmChoice choose_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, 
   }
   if (c.kernel == GEMM_NONE && c.general.bn) c.kernel = GEMM_GENERAL;
   return c;
+}
+
+// The last choices of this thread: a search looks at some 200 schedules (1 to 4 us), and a model asks for the same few over and
+// over.  32 sets of four entries, replaced in turn; the set is taken from the top bits of a multiplicative hash, because
+// N and K of real layers are multiples of 64 and agree in all their low bits.
+GemmChoice choose_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, size_t ws_bytes) {
+  struct Key {
+    int64_t M, N, K;
+    size_t ws_bytes;
+    int epi, head_size, neox, tile_cfg, dev, used;
+  };
+  struct Entry { Key key; GemmChoice choice; };
+  static thread_local Entry memo[32][4];
+  static thread_local unsigned char next[32];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); dev = -1; }
+  const Key key = {M, N, K, ws_bytes, epi, head_size, neox, tile_cfg, dev, 1};
+  uint64_t h = 0;
+  for (uint64_t v : {(uint64_t)M, (uint64_t)N, (uint64_t)K, (uint64_t)epi + 8 * (uint64_t)(uint32_t)tile_cfg}) h = ((h ^ v) * 0x9E3779B97F4A7C15ull) ^ (h >> 32);
+  const int set = (int)(h >> 59);
+  for (Entry& e : memo[set])
+    if (e.key.used && e.key.M == M && e.key.N == N && e.key.K == K && e.key.ws_bytes == ws_bytes && e.key.epi == epi &&
+        e.key.head_size == head_size && e.key.neox == neox && e.key.tile_cfg == tile_cfg && e.key.dev == dev)
+      return e.choice;
+  Entry& e = memo[set][next[set]];
+  next[set] = (unsigned char)((next[set] + 1) & 3);
+  e.key.used = 0;
+  e.choice = search_gemm(epi, M, N, K, head_size, neox, tile_cfg, ws_bytes);
+  e.key = key;
+  return e.choice;
 }
 
 // Arrivals the row-parallel kernel of a rank counts for the rank that owns
@@ -514,6 +547,8 @@ extern "C" int sb200_gemm_plan(int epilogue, int64_t T, int64_t N, int64_t K, in
   write_plan(p, out);
   return p.bn ? SB200_OK : SB200_ERR_UNSUPPORTED;
 }
+
+extern "C" int64_t sb200_gemm_choices_made(void) { return choices_made; }
 
 // The launch sb200_gemm_colpar makes of a bf16 / fp16 problem: out[0] = kernel, then its schedule (see the header).
 extern "C" int sb200_gemm_launch(int epilogue, int64_t T, int64_t N, int64_t K, int head_size, int is_neox, int tile_cfg,

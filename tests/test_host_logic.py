@@ -653,3 +653,25 @@ def test_autotune_candidates_are_distinct_launches():
         cfgs = D._candidates(kind, T, N, K, 128)
         launches = [tuple(D.gemm_launch(epi, T, N, K, 128, c).items()) for c in cfgs]
         assert len(set(launches)) == len(cfgs) and any(x[0] == ("kernel", "swapped") for x in launches)
+
+
+@pytest.mark.parametrize("tp", [1, 8])
+@pytest.mark.parametrize("H,I,qkv", [(4096, 14336, 6144), (8192, 28672, 10240)])
+def test_the_schedules_of_a_layer_are_searched_once(H, I, qkv, tp):
+    """The projections of a layer and the vocabulary, for one batch size after the other: the second pass over them
+    finds every choice (N and K of real layers are all multiples of 64)."""
+    from sarathi_serve_b200 import _native as N_, dense_ops as D
+    made = N_.lib().sb200_gemm_choices_made
+    problems = [(1, qkv // tp, H), (0, H, H // tp), (2, 2 * I // tp, H), (0, H, I // tp), (0, 128256 // tp, H)]
+    for T in (1, 8, 61, 64, 96, 256, 512, 777, 1024, 2048):
+        first = [D.gemm_launch(epi, T, N, K) for epi, N, K in problems]
+        before = made()
+        for _ in range(3):
+            assert [D.gemm_launch(epi, T, N, K) for epi, N, K in problems] == first
+        assert made() == before, T
+    # another workspace, head layout or configuration is another problem
+    before = made()
+    D.gemm_launch(1, 300, 768, 4096, workspace_bytes=0)
+    D.gemm_launch(1, 300, 768, 4096, is_neox=False)
+    D.gemm_launch(1, 300, 768, 4096, tile_cfg=128)
+    assert made() >= before + (3 if (H, tp) == (4096, 1) else 0)
