@@ -10,7 +10,7 @@
 // How:
 //   * NACC = 2 accumulators per CTA share the tokens of a stage: gate and up rows (EPI_SILU_MUL), the first and the second
 //     halves of 128 / (head_size / 2) heads (EPI_ROTARY), so that the two values a thread combines sit in the same
-//     lane; or simply 256 columns (EPI_STORE, large batches).
+//     lane.  EPI_STORE has one accumulator; two (256 columns) only by explicit configuration, for the autotuner.
 //   * Few tiles: K is cut over a cluster of `split` CTAs.  Every CTA sends the others the tokens they finish through
 //     distributed shared memory and sums its own tokens in the order of the k-ranges: no workspace, nothing that two
 //     streams could share, and a result that does not depend on timing.
@@ -361,7 +361,11 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 static int swap_clusters(int split, int ew) {
   static std::atomic<int> cache[16][2][9];  // [device][ew][split]; 0 = not asked yet
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16 || split < 1 || split > 8) return sm_count() / (split < 1 ? 1 : split);
+  if (split < 2 || split > 8) return sm_count();
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) {  // planning without a device: as max_coresident_clusters
+    (void)cudaGetLastError();
+    return sm_count() / split * 3 / 4;
+  }
   std::atomic<int>& c = cache[dev][ew == 4 ? 0 : 1][split];
   int n = c.load(std::memory_order_relaxed);
   if (n > 0) return n;
@@ -389,7 +393,7 @@ static int swap_clusters(int split, int ew) {
 }
 
 // A plan for `nacc` accumulators, t_tiles token tiles and `split` CTAs per tile; false when it does not fit.
-static bool swap_plan(int epi, int64_t M, int64_t N, int64_t K, int head_size, int nacc, int t_tiles, int split, SwapPlan* p) {
+static bool swap_plan(int64_t M, int64_t N, int64_t K, int head_size, int nacc, int t_tiles, int split, SwapPlan* p) {
   const int sms = sm_count();
   const int64_t per = (M + t_tiles - 1) / t_tiles;
   const int64_t nt = (per + 15) / 16 * 16;
@@ -471,20 +475,21 @@ static bool search_swap(int epi, int64_t M, int64_t N, int64_t K, int head_size,
     const int nt = tile_cfg % 1000, mode = (tile_cfg / 1000) % 100, split = tile_cfg / 100000 > 1 ? tile_cfg / 100000 : 1;
     if (nt < 16 || nt > 256 || (mode == 7 && epi != EPI_STORE)) return false;
     *cost = 0.0;
-    return swap_plan(epi, M, N, K, head_size, mode == 7 ? 1 : 2, (int)((M + nt - 1) / nt), split, best);
+    return swap_plan(M, N, K, head_size, mode == 7 ? 1 : 2, (int)((M + nt - 1) / nt), split, best);
   }
   const int64_t t_min = (M + 255) / 256, t_max = (M + 15) / 16 < t_min + 12 ? (M + 15) / 16 : t_min + 12;
-  // (EPI_STORE: with two accumulators no shape below 1300 tokens was faster, and 777 x 4096 x 4096 took 35 us against 24)
-  for (int nacc = epi == EPI_STORE ? 1 : 2, last = nacc; nacc <= last; ++nacc)
-    for (int64_t t = t_min; t <= t_max; ++t)
-      for (int s = 1; s <= 8; ++s) {
-        SwapPlan p;
-        if (!swap_plan(epi, M, N, K, head_size, nacc, (int)t, s, &p)) continue;
-        if (s > 1 && ((int64_t)p.w_tiles * t * s > sm_count() || p.k_blocks / s < 4)) break;
-        if (s > 1 && (int64_t)p.w_tiles * t > swap_clusters(s, p.ew)) continue;  // one round of clusters
-        const double c = swap_cost(epi, N, K, p);
-        if (c < *cost) { *cost = c; *best = p; }
-      }
+  // one accumulator for EPI_STORE, always: with two no shape below 1300 tokens was faster, and 777 x 4096 x 4096 took 35 us
+  // against 24; beyond that the general kernel has most shapes
+  const int nacc = epi == EPI_STORE ? 1 : 2;
+  for (int64_t t = t_min; t <= t_max; ++t)
+    for (int s = 1; s <= 8; ++s) {
+      SwapPlan p;
+      if (!swap_plan(M, N, K, head_size, nacc, (int)t, s, &p)) continue;
+      if (s > 1 && ((int64_t)p.w_tiles * t * s > sm_count() || p.k_blocks / s < 4)) break;
+      if (s > 1 && (int64_t)p.w_tiles * t > swap_clusters(s, p.ew)) continue;  // one round of clusters
+      const double c = swap_cost(epi, N, K, p);
+      if (c < *cost) { *cost = c; *best = p; }
+    }
   return *cost < 1e30;
 }
 
