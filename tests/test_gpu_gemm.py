@@ -292,12 +292,15 @@ def test_linear_few_columns(dtype, T, N, K):
     assert rel_err(got.float(), r.double() + (ref + b.double()).to(dtype).double()) <= GEMM_TOL[dtype]
 
 
-# The same kernel on larger, ragged batches: token tiles of 16..256, one and two accumulators, K over a cluster, several
-# rounds of tiles per CTA with one and with two sets of accumulators.
+# The same kernel on larger, ragged batches: token tiles of 16..176 (the tokens are spread evenly over the tiles), one and two
+# accumulators, K over a cluster.  More than one round of tiles only for 6016 and 7064 with 513 tokens, both on two sets of
+# accumulators; the other rounds: test_swapped_tiles_over_several_rounds.
 @pytest.mark.parametrize("cfg", [6016, 6112, 6128, 6256, 7064, 7256, 206064, 807032, 306176])
 @pytest.mark.parametrize("T,N,K", [(65, 256, 512), (129, 200, 1000), (300, 1000, 512), (513, 4096, 576)])
 def test_linear_swapped_tiles(cfg, T, N, K):
     from sarathi_serve_b200 import dense_ops
+    p = dense_ops.gemm_launch(0, T, N, K, tile_cfg=cfg)
+    assert p["kernel"] == "swapped" and p["k_parts"] == max(1, cfg // 100000)
     x, w = _rand((T, K), torch.bfloat16, T + N).cuda(), _rand((N, K), torch.bfloat16, N + K, 0.05).cuda()
     b, r = _rand((N,), torch.bfloat16, 3).cuda(), _rand((T, N), torch.bfloat16, 4).cuda()
     out = dense_ops.linear(x, w, tile_n=cfg)
@@ -313,6 +316,7 @@ def test_linear_swapped_tiles(cfg, T, N, K):
 def test_linear_rotary_and_silu_swapped_tiles(cfg, T, nq, nkv, hd):
     from sarathi_serve_b200 import dense_ops
     N, K = (nq + 2 * nkv) * hd, 320
+    assert all(dense_ops.gemm_launch(epi, T, N, K, hd, cfg)["kernel"] == "swapped" for epi in (1, 2))
     x, w = _rand((T, K), torch.float16, T).cuda(), _rand((N, K), torch.float16, N, 0.05).cuda()
     pos = torch.randint(0, 2048, (T,), generator=torch.Generator().manual_seed(5)).cuda()
     cs = O.cos_sin_cache(hd, hd, 2048, 10000.0, torch.float16).cuda()
@@ -326,6 +330,64 @@ def test_linear_rotary_and_silu_swapped_tiles(cfg, T, nq, nkv, hd):
     acts = [dense_ops.linear_silu_mul(x, w, tile_n=c) for c in (cfg, 128)]
     _check_status()
     assert rel_err(acts[0], acts[1]) <= 2e-2
+
+
+# Several rounds of tiles per CTA, on one set of accumulators (a tile is finished before the next one's MMAs) and on two (its
+# epilogue under the next tile's loop), three and more uses of a set; the largest token tiles.
+@pytest.mark.parametrize("epi,T,cols,K,cfg,tokens,sets,rounds", [
+    ("silu", 300, 14336, 128, 6160, 160, 1, 2), ("silu", 800, 14336, 64, 6160, 160, 1, 4), ("silu", 896, 14336, 64, 6128, 128, 2, 6),
+    ("silu", 16, 19100, 64, 6016, 16, 2, 2), ("silu", 512, 200, 264, 6256, 256, 1, 1), ("silu", 200, 14336, 192, 6208, 208, 1, 1),
+    ("store", 800, 25600, 64, 6160, 160, 1, 4), ("store", 1120, 15300, 72, 6112, 112, 2, 5), ("store", 512, 1000, 520, 6256, 256, 1, 1),
+    ("store", 2048, 8000, 64, 7256, 256, 2, 4), ("store", 200, 300, 264, 7208, 208, 1, 1),
+    ("rotary", 800, 15360, 64, 6160, 160, 1, 3), ("rotary", 1120, 15360, 64, 6112, 112, 2, 5), ("rotary", 512, 768, 320, 6256, 256, 1, 1),
+    ("rotary", 200, 1024, 264, 6208, 208, 1, 1)])
+def test_swapped_tiles_over_several_rounds(epi, T, cols, K, cfg, tokens, sets, rounds):
+    from sarathi_serve_b200 import dense_ops
+    dtype, hd, u = torch.float16, 128, 2.0 ** -11
+    N = 2 * cols if epi == "silu" else cols
+    p = dense_ops.gemm_launch({"store": 0, "rotary": 1, "silu": 2}[epi], T, N, K, hd, cfg)
+    assert (p["kernel"], p["tokens"], p["accumulator_sets"], p["rounds"]) == ("swapped", tokens, sets, rounds)
+    x, w = _rand((T, K), dtype, T + K).cuda(), _rand((N, K), dtype, N + K, 0.1).cuda()
+    y, absum = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    sums = (K + 64) * 2.0 ** -24 * absum  # products and sums in fp32
+    if epi == "store":
+        out = dense_ops.linear(x, w, tile_n=cfg)
+        _check_status()
+        assert bool(((out.double() - y).abs() <= _bf_bound(y, absum, K, dtype)).all())
+        return
+    if epi == "silu":
+        out = dense_ops.linear_silu_mul(x, w, tile_n=cfg)
+        _check_status()
+        g, up = y[:, :cols], y[:, cols:]
+        f = g * torch.sigmoid(g)
+        # gate rounded before silu (slope at most 1.1), silu, up and the product rounded; 5 % for the terms of higher order
+        bound = 1.1 * (u * g.abs() + sums[:, :cols]) * up.abs() + f.abs() * (3.2 * u * up.abs() + sums[:, cols:])
+        assert bool(((out.double() - f * up).abs() <= 1.05 * bound + 1e-6).all())
+        return
+    heads = cols // hd
+    nkv = heads // 6
+    rot, page = (heads - nkv) * hd, 16
+    pos = torch.randint(0, 2048, (T,), generator=torch.Generator().manual_seed(5)).cuda()
+    cs = O.cos_sin_cache(hd, hd, 2048, 10000.0, dtype).cuda()
+    cache = torch.zeros((T + page - 1) // page, 2, page, nkv, hd, dtype=dtype, device="cuda")
+    t = torch.arange(T, device="cuda")
+    slots = t // page * 2 * page + t % page
+    out = dense_ops.linear_rotary(x, w, pos, cs, hd, rot, True, tile_n=cfg, kv_cache=cache, kv_slots=slots, num_kv_heads=nkv)
+    _check_status()
+    c, s = cs[pos].double()[:, None, :hd // 2], cs[pos].double()[:, None, hd // 2:]
+
+    def halves(m):
+        m = m[:, :rot].view(T, -1, hd)
+        return m[..., :hd // 2], m[..., hd // 2:]
+    (a, b), (ea, eb) = halves(y), halves(sums)
+    want = torch.cat([a * c - b * s, b * c + a * s], -1).view(T, rot)
+    # both inputs, both products and the result rounded
+    ra, rb = 2 * u * a.abs() + ea, 2 * u * b.abs() + eb
+    bound = torch.cat([ra * c.abs() + rb * s.abs(), rb * c.abs() + ra * s.abs()], -1).view(T, rot) + u * want.abs()
+    assert bool(((out[:, :rot].double() - want).abs() <= 1.05 * bound + 1e-6).all())
+    assert bool(((out[:, rot:].double() - y[:, rot:]).abs() <= _bf_bound(y, absum, K, dtype)[:, rot:]).all())
+    flat, kv = cache.view(-1, nkv * hd), nkv * hd
+    assert torch.equal(flat[slots], out[:, rot - kv:rot]) and torch.equal(flat[slots + page], out[:, rot:rot + kv])
 
 
 # Explicit configurations that do not fit are refused, not run as something else: too few and too many tokens a tile, more
