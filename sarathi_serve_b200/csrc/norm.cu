@@ -12,13 +12,17 @@ namespace sb200 {
 
 constexpr int kNormMaxVec = 4;  // most 16-byte vectors cached per thread
 
-// VEC: 16-byte vectors a thread holds (registers decide how many rows an SM works on: 1 whenever a row has at most 512
-// of them), or 0 for the generic path.
-template <typename T, bool ADD, int VEC>
+// VEC: 16-byte vectors a thread holds, or 0 for the generic path.  Bound by memory, and by how many rows an SM has in flight.
+// EARLY: the weights are loaded with the row, so that their latency hides behind its own; they then stay in registers over the
+// reduction.  Good for up to two vectors and for a batch of at most a row per SM (64 rows of 24576: 4.5 -> 3.6 us); with
+// more of both it costs the SM a resident row (8192 rows of 16384: 139 us against 96).
+// early_next: let the next kernel start under this one.
+template <typename T, bool ADD, int VEC, bool EARLY>
 __global__ void __launch_bounds__(1024)
 rms_norm_kernel(T* out, T* resid_out, const T* x, const T* resid,
-                const T* w, float eps, int H) {
-  grid_dependency_begin();
+                const T* w, float eps, int H, int early_next) {
+  if (early_next) ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
   __shared__ float red[33];
   constexpr int N = Vec16<T>::N;
   const int64_t row = blockIdx.x;
@@ -29,14 +33,14 @@ rms_norm_kernel(T* out, T* resid_out, const T* x, const T* resid,
   float ss = 0.f;
 
   if constexpr (VEC > 0) {
-    Vec16<T> cache[VEC], wv[VEC];
+    Vec16<T> cache[VEC], wv[EARLY ? VEC : 1];
     const int nvec = H / N;
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int v = i * blockDim.x + threadIdx.x;
       if (v < nvec) {
         cache[i] = ld16(xr + v * N);
-        wv[i] = ld16(w + v * N);  // (needed after the reduction: its latency hides behind that of the row)
+        if constexpr (EARLY) wv[i] = ld16(w + v * N);
         if constexpr (ADD) {
           Vec16<T> r = ld16(rr + v * N);
 #pragma unroll
@@ -57,10 +61,12 @@ rms_norm_kernel(T* out, T* resid_out, const T* x, const T* resid,
     for (int i = 0; i < VEC; ++i) {
       const int v = i * blockDim.x + threadIdx.x;
       if (v < nvec) {
-        Vec16<T> o;
+        Vec16<T> o, wi;
+        if constexpr (EARLY) wi = wv[i];
+        else wi = ld16(w + v * N);
 #pragma unroll
         for (int j = 0; j < N; ++j)
-          o.v[j] = DT<T>::from_f(rt<T>(DT<T>::to_f(cache[i].v[j]) * inv) * DT<T>::to_f(wv[i].v[j]));
+          o.v[j] = DT<T>::from_f(rt<T>(DT<T>::to_f(cache[i].v[j]) * inv) * DT<T>::to_f(wi.v[j]));
         st16(orow + v * N, o);
       }
     }
@@ -92,18 +98,25 @@ static int launch_norm(void* out, void* resid_out, const void* x, const void* re
   if (vec) {
     const int64_t nvec = H / N;
     // fewest vectors per thread that keep the CTA at >= 128 threads when possible
-    while (per < kNormMaxVec && (nvec + per - 1) / per > 512) per *= 2;
+    while (per < kNormMaxVec && (nvec + per - 1) / per > 512) ++per;
     int64_t t = (nvec + per - 1) / per;
     t = (t + 31) / 32 * 32;
     if (t > 1024) vec = false;
     threads = (int)t;
   }
   if (!vec) threads = (int)((H < 1024 ? (H + 31) / 32 * 32 : 1024));
-  const dim3 grid((unsigned)T_);
-  auto kern = !vec ? rms_norm_kernel<T, ADD, 0> : per == 1 ? rms_norm_kernel<T, ADD, 1>
-              : per == 2 ? rms_norm_kernel<T, ADD, 2> : rms_norm_kernel<T, ADD, kNormMaxVec>;
-  launch_dependent(kern, grid, dim3((unsigned)threads), 0, s, (T*)out, (T*)resid_out, (const T*)x, (const T*)resid, (const T*)w,
-                   eps, (int)H);
+  const bool few = T_ <= sm_count();
+  // Signalling the next kernel takes 1.1 ns per CTA of the grid, whatever the CTA does (8192 rows of 64: 9.0 us against 6.0 without),
+  // and CTAs that wait in the slots a row or two leave free unbalance the launch they belong to (512 rows of 5120 after one
+  // another: 4.9 us against 4.4).  So only where a row is large enough to hide the first and fills the SM's threads, or the
+  // batch is small.
+  const int early_next = few || (vec && per <= 2 && threads >= 448) ? 1 : 0;
+  auto kern = !vec ? rms_norm_kernel<T, ADD, 0, false> : per == 1 ? rms_norm_kernel<T, ADD, 1, true>
+              : per == 2 ? rms_norm_kernel<T, ADD, 2, true>
+              : per == 3 ? (few ? rms_norm_kernel<T, ADD, 3, true> : rms_norm_kernel<T, ADD, 3, false>)
+                         : (few ? rms_norm_kernel<T, ADD, kNormMaxVec, true> : rms_norm_kernel<T, ADD, kNormMaxVec, false>);
+  launch_dependent(kern, dim3((unsigned)T_), dim3((unsigned)threads), 0, s, (T*)out, (T*)resid_out, (const T*)x, (const T*)resid,
+                   (const T*)w, eps, (int)H, early_next);
   SB_CHECK_LAUNCH("rms_norm_kernel");
   return SB200_OK;
 }

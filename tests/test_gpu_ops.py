@@ -201,6 +201,39 @@ def test_vocab_parallel_embedding_module_tp1():
         ps.destroy_model_parallel()
 
 
+# One to four 16-byte vectors per thread, the weights loaded with the row (up to a row per SM, or up to two vectors) or after the
+# sum, more vectors than threads hold, and rows that are no multiple of 16 bytes.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T", [1, 148, 149, 301])
+@pytest.mark.parametrize("H", [2056, 5120, 9216, 12288, 16384, 33024, 1001])
+def test_norm_rows_of_every_width(dtype, T, H):
+    from sarathi_serve_b200 import layernorm_ops
+    g = torch.Generator().manual_seed(T + H)
+    x, r = torch.randn(T, H, generator=g).to(dtype).cuda(), torch.randn(T, H, generator=g).to(dtype).cuda()
+    w = (1 + 0.1 * torch.randn(H, generator=g)).to(dtype).cuda()
+    # the factor 1 / rms is good to a few roundings of fp32; the row and the product are each rounded to the type
+    u = {torch.float32: 2.0 ** -24, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+
+    def check(out, z):
+        want = z.double() * torch.rsqrt(z.double().square().mean(-1, keepdim=True) + 1e-5)
+        bound = (2.1 * u + 16 * 2.0 ** -24) * (want * w.double()).abs() + 1e-7
+        assert bool(((out.double() - want * w.double()).abs() <= bound).all())
+    out, guard = _canary((T, H), dtype)
+    layernorm_ops.rms_norm(out, x, w, 1e-5)
+    guard()
+    check(out, x)
+    out, guard = _canary((T, H), dtype)
+    z, guard_z = _canary((T, H), dtype)
+    layernorm_ops.fused_add_rms_norm(out, z, x, r, w, 1e-5)
+    guard()
+    guard_z()
+    assert torch.equal(z, x + r)
+    check(out, z)
+    again = torch.empty_like(x)
+    layernorm_ops.fused_add_rms_norm(again, r, x, r, w, 1e-5)  # the residual in place
+    assert torch.equal(r, z) and torch.equal(again, out)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T", [3, 600])  # (600: block alignment over a cluster)
 def test_chain_of_small_kernels_on_shared_buffers(dtype, T):
