@@ -325,7 +325,9 @@ moe_align_single_kernel(const void* ids, int itype, int64_t numel, int E, int bl
 // steps instead of 48), 8192 of 16 17.3 -> 6.6 us, 1800 of 128 14.5 -> 10.8 us.
 // smem ints: cnt[32][E] | cumsum[E+1] | totals[E] | before[E]
 constexpr int kAlignCluster = 8;
-constexpr int64_t kAlignClusterSlots = 1024;  // (2048 slots of 8 experts: 5.3 us in one CTA, 5.4 us in a cluster; 4096: 7.8, 5.6)
+// Few experts leave a single CTA fast for longer: 2048 slots of 1 / 8 / 64 experts take 4.5 / 5.9 / 11.9 us in one CTA and 4.9 / 5.5 / 8.4 us
+// in a cluster, 1025 slots 4.4 / 5.1 / 9.5 and 4.8 / 5.3 / 8.0 us.
+static bool align_over_cluster(int64_t numel, int E) { return numel > (E < 8 ? 2048 : E < 16 ? 1280 : 1024); }
 __global__ void __cluster_dims__(kAlignCluster, 1, 1) __launch_bounds__(1024)
 moe_align_cluster_kernel(const void* ids, int itype, int64_t numel, int E, int block, int32_t* sorted,
                          int64_t sorted_cap, int32_t* expert_ids, int64_t expert_cap, int32_t* num_post_pad) {
@@ -515,7 +517,7 @@ extern "C" int sb200_moe_align_block_size(const void* topk_ids, int ids_itype, i
       return SB200_ERR_UNSUPPORTED;
     }
     const size_t smem_cluster = smem + 2 * (size_t)E * sizeof(int);
-    if (numel > kAlignClusterSlots && smem_cluster <= 200 * 1024) {
+    if (align_over_cluster(numel, E) && smem_cluster <= 200 * 1024) {
       if (smem_cluster > 40 * 1024)
         SB_CUDA(cudaFuncSetAttribute(moe_align_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cluster));
       launch_dependent(moe_align_cluster_kernel, kAlignCluster, 1024, smem_cluster, s, topk_ids, ids_itype, numel, E, block_size,

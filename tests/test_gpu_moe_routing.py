@@ -113,9 +113,11 @@ def test_moe_align_block_size(itype, T, k, E, block, scratch):
         assert torch.equal(re_[:npp // block], e[:npp // block])
 
 
-# One slot more than a single CTA takes, segments that end inside a warp's step, one expert, more experts than threads a
-# CTA of the cluster scans at once, and all slots in the last expert.
-@pytest.mark.parametrize("T,k,E,block", [(1024, 1, 8, 64), (1025, 1, 1, 16), (2049, 1, 200, 16), (8192, 6, 128, 128), (1500, 3, 1100, 7)])
+# The most slots of a single CTA and one more (its limit grows as experts become few), segments that end inside a warp's step, one
+# expert, more experts than threads a CTA of the cluster scans at once, and all slots in the last expert.
+@pytest.mark.parametrize("T,k,E,block", [(1024, 1, 8, 64), (1025, 1, 1, 16), (2049, 1, 200, 16), (8192, 6, 128, 128), (1500, 3, 1100, 7),
+                                         (2048, 1, 1, 16), (2049, 1, 1, 16), (1280, 1, 8, 16), (1281, 1, 8, 16), (1024, 1, 16, 16),
+                                         (1025, 1, 16, 16)])
 @pytest.mark.parametrize("skew", [False, True])
 def test_align_over_a_cluster(T, k, E, block, skew):
     g = torch.Generator().manual_seed(T)
