@@ -557,7 +557,7 @@ extern "C" int sb200_gemm_launch(int epilogue, int64_t T, int64_t N, int64_t K, 
                    epilogue <= SB200_EPI_SILU_MUL, "gemm_launch: bad arguments");
   const int epi = epi_of(epilogue);
   for (int i = 0; i < 13; ++i) out[i] = 0;
-  if (tile_cfg == 0 && narrow_fits(epi, N, K)) {
+  if (tile_cfg == 0 && narrow_fits(epi, T, N, K)) {
     out[0] = 2;
     return SB200_OK;
   }

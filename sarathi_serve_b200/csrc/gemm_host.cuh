@@ -50,9 +50,9 @@ struct SwapPlan {
 bool plan_swap(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, SwapPlan* plan, double* clocks);
 int run_gemm_swap(int dtype, int epi, const SwapPlan& plan, const void* x, int64_t ldx, const void* w, int64_t ldw,
                   const GemmArgs& g, cudaStream_t s);
-// At most 16 output columns (gemm_narrow.cu).  `fits`: the shape; `*done` = false: the operands' rows cannot be read in 16-byte
+// At most 16 output columns and not too many tokens (gemm_narrow.cu).  `fits`: the shape; `*done` = false: the operands' rows cannot be read in 16-byte
 // pieces, nothing was launched.
-bool narrow_fits(int epi, int64_t N, int64_t K);
+bool narrow_fits(int epi, int64_t M, int64_t N, int64_t K);
 int run_gemm_narrow(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g,
                     cudaStream_t s, bool* done);
 // Which tensor-core kernel runs a problem, with its schedule.

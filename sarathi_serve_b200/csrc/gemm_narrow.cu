@@ -63,23 +63,32 @@ gemm_narrow_kernel(const T* x, int64_t ldx, const T* w, int64_t ldw, const GemmA
   }
 }
 
+// Tokens of a CTA: eight reuse the weights most; two while that still leaves SMs without a CTA.
+static int narrow_rows(int64_t M) { return M <= 2 * sm_count() ? 2 : 8; }
+
 template <typename T>
 static cudaError_t launch_narrow(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g, cudaStream_t s) {
-  const unsigned groups = (unsigned)((g.N + 7) / 8);
-  // eight tokens per CTA reuse the weights most; two while that still leaves SMs without a CTA
-  if (g.M <= 2 * sm_count())
-    return launch_dependent(gemm_narrow_kernel<T, 2>, dim3((unsigned)((g.M + 1) / 2), groups), dim3(kNarrowWarps * 32), 0, s,
-                            (const T*)x, ldx, (const T*)w, ldw, g);
-  return launch_dependent(gemm_narrow_kernel<T, 8>, dim3((unsigned)((g.M + 7) / 8), groups), dim3(kNarrowWarps * 32), 0, s,
-                          (const T*)x, ldx, (const T*)w, ldw, g);
+  const int rows = narrow_rows(g.M);
+  const dim3 grid((unsigned)((g.M + rows - 1) / rows), (unsigned)((g.N + 7) / 8)), block(kNarrowWarps * 32);
+  return launch_dependent(rows == 2 ? gemm_narrow_kernel<T, 2> : gemm_narrow_kernel<T, 8>, grid, block, 0, s, (const T*)x, ldx,
+                          (const T*)w, ldw, g);
 }
 
-bool narrow_fits(int epi, int64_t N, int64_t K) { return epi == EPI_STORE && N <= kNarrowMaxCols && K % 8 == 0; }
+// An SM holds one CTA of eight tokens, so the time goes in rounds of 148 of them (8 columns, K = 4096: 1184 tokens 6.1 us, 1200
+// 10.8, 2400 15.8, 4096 21 us), while the tensor-core kernels take 10 to 12 us for all of these: one round, and a second where
+// K is long enough to make theirs slow and short enough to keep this one fast (1200 tokens, K = 512: 5.7 us against 5.2,
+// 1024: 5.9 / 10.4, 4096: 10.8 / 11.5, 6144: 13.8 / 12.3 us).
+bool narrow_fits(int epi, int64_t M, int64_t N, int64_t K) {
+  if (epi != EPI_STORE || N > kNarrowMaxCols || K % 8) return false;
+  const int rows = narrow_rows(M);
+  const int64_t ctas = (M + rows - 1) / rows * ((N + 7) / 8), sms = sm_count();
+  return rows == 2 || ctas <= sms || (ctas <= 2 * sms && K >= 1024 && K <= 4096);
+}
 
 int run_gemm_narrow(int dtype, int epi, const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmArgs& g,
                     cudaStream_t s, bool* done) {
   // rows that the 16-byte loads can read; anything else is left to the tensor-core kernel, which also words the errors
-  *done = narrow_fits(epi, g.N, g.K) && (dtype == SB200_BF16 || dtype == SB200_F16) && ldx >= g.K && ldw >= g.K &&
+  *done = narrow_fits(epi, g.M, g.N, g.K) && (dtype == SB200_BF16 || dtype == SB200_F16) && ldx >= g.K && ldw >= g.K &&
           ldx % 8 == 0 && ldw % 8 == 0 && aligned16(x) && aligned16(w);
   if (!*done) return SB200_OK;
   SB_CUDA(dtype == SB200_BF16 ? launch_narrow<__nv_bfloat16>(x, ldx, w, ldw, g, s) : launch_narrow<__half>(x, ldx, w, ldw, g, s));

@@ -638,6 +638,9 @@ def test_swapped_launches_are_consistent(T, epi, N, K):
 def test_which_kernel_a_projection_takes():
     from sarathi_serve_b200 import dense_ops as D
     assert D.gemm_launch(0, 1024, 8, 4096)["kernel"] == "narrow" and D.gemm_launch(0, 1024, 16, 4096)["kernel"] == "narrow"
+    assert D.gemm_launch(0, 1184, 8, 64)["kernel"] == "narrow" and D.gemm_launch(0, 592, 16, 14336)["kernel"] == "narrow"
+    for T, N, K in ((1185, 8, 64), (593, 9, 512), (1185, 8, 4160), (2369, 8, 4096), (65536, 1, 1024)):  # more rounds than pay off
+        assert D.gemm_launch(0, T, N, K)["kernel"] != "narrow", (T, N, K)
     assert D.gemm_launch(0, 4, 17, 4096)["kernel"] == "swapped"
     assert D.gemm_launch(0, 4, 8, 4100)["kernel"] == "swapped"                       # rows that are no multiple of 16 bytes
     assert D.gemm_launch(1, 4, 768, 4096, is_neox=False)["kernel"] == "general"      # pairs of a GPT-J head sit side by side
