@@ -268,19 +268,29 @@ static GemmChoice search_gemm(int epi, int64_t M, int64_t N, int64_t K, int head
     tile_cfg = 0;
     swapped_only = false;
   }
-  if (!swapped_only && (tile_cfg != 0 || M > 64 || epi == EPI_PUSH))
-    c.general = plan_gemm(epi, M, N, K, head_size, tile_cfg, ws_bytes, neox);
-  if (epi != EPI_PUSH && (tile_cfg == 0 || swapped_only)) {
-    // Up to 64 tokens always (8 tokens x 28672 x 4096: 42 us against 66, 64 tokens: 43 against 56); beyond that where the
-    // estimate is an eighth better: ragged batches (300 tokens x 28672 x 4096: 78 us against 100) and few tiles
-    // (512 x 768 x 4096: 15.5 against 22), while whole 256-row tiles of CTA pairs need half of the operand traffic
-    // (512 tokens x 28672 x 4096: 97 us there, 115 here).
-    double clocks = 0.0;
-    if (plan_swap(epi, M, N, K, head_size, neox, tile_cfg, &c.swapped, &clocks) &&
-        (swapped_only || M <= 64 || clocks < 0.87 * gemm_plan_clocks(epi, N, K, c.general)))
-      c.kernel = GEMM_SWAPPED;
-    else if (!swapped_only && M <= 64)  // (a head layout the swapped kernel does not take)
-      c.general = plan_gemm(epi, M, N, K, head_size, tile_cfg, ws_bytes, neox);
+  double clocks = 0.0;
+  const bool swapped = epi != EPI_PUSH && (tile_cfg == 0 || swapped_only) && plan_swap(epi, M, N, K, head_size, neox, tile_cfg, &c.swapped, &clocks);
+  if (swapped_only) {
+    if (swapped) c.kernel = GEMM_SWAPPED;
+    return c;
+  }
+  // Up to 64 tokens (8 tokens x 28672 x 4096: 41 us against 59, 64 tokens x 4096 x 14336: 28.5 against 33.6), except with more
+  // tiles than SMs where the last round is nearly empty or the rings are too shallow for the walk (plain, 8 tokens x 19072 x 4096,
+  // 149 tiles: 40 us against 31; 61 tokens x 28672 x 4096: 48.4 / 43.7, x 128256: 177 / 172; but 16 tokens x 128256 x 1024: 42 / 47).
+  const bool walks = swapped && c.swapped.split == 1 && (int64_t)c.swapped.w_tiles * c.swapped.t_tiles > c.swapped.grid;
+  if (swapped && M <= 64 && !walks) {
+    c.kernel = GEMM_SWAPPED;
+    return c;
+  }
+  c.general = plan_gemm(epi, M, N, K, head_size, tile_cfg, ws_bytes, neox);
+  if (swapped) {
+    // Beyond 64 tokens where the estimate is an eighth better: ragged batches (300 tokens x 28672 x 4096: 78 us against 100)
+    // and few tiles (512 x 768 x 4096: 15.5 against 22), while whole 256-row tiles of CTA pairs need half of the operand
+    // traffic (512 tokens x 28672 x 4096: 97 us there, 115 here).  The walk of a small batch: the ratios of the estimates where
+    // the measured times are equal (the general kernel's is low for batches this small, most with the fused epilogues).
+    const double other = gemm_plan_clocks(epi, N, K, c.general);
+    const double level = epi == EPI_STORE ? 1.08 : epi == EPI_ROTARY ? 1.15 : 1.38;
+    if (M <= 64 ? swap_walk_clocks(epi, K, c.swapped) <= level * other : clocks < 0.87 * other) c.kernel = GEMM_SWAPPED;
   }
   if (c.kernel == GEMM_NONE && c.general.bn) c.kernel = GEMM_GENERAL;
   return c;

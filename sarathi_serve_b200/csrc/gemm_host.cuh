@@ -48,6 +48,8 @@ struct SwapPlan {
 };
 // tile_cfg 0: the cheapest plan and its estimated clocks; else the plan of that configuration (MODE 6|7).  False: none.
 bool plan_swap(int epi, int64_t M, int64_t N, int64_t K, int head_size, int neox, int tile_cfg, SwapPlan* plan, double* clocks);
+// Clocks of a projection of up to 64 tokens whose CTAs walk several rounds of whole tiles.
+double swap_walk_clocks(int epi, int64_t K, const SwapPlan& plan);
 int run_gemm_swap(int dtype, int epi, const SwapPlan& plan, const void* x, int64_t ldx, const void* w, int64_t ldw,
                   const GemmArgs& g, cudaStream_t s);
 // At most 16 output columns and not too many tokens (gemm_narrow.cu).  `fits`: the shape; `*done` = false: the operands' rows cannot be read in 16-byte

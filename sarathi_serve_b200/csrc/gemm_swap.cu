@@ -430,7 +430,7 @@ static bool swap_plan(int64_t M, int64_t N, int64_t K, int head_size, int nacc, 
 
 // Estimated SM clocks.  The constants are fitted to the kernel's times over 8 .. 2048 tokens of the projections of 8B and
 // 70B layers, whole and at 1/8 of the width (most within 15 %).
-static double swap_cost(int epi, int64_t N, int64_t K, const SwapPlan& p) {
+static double swap_per_kb(int epi, const SwapPlan& p) {
   const int sms = sm_count();
   const double stage = p.nacc * kSwapTileBytes + p.act_rows * kBK * 2;
   double per_kb = 4.0 * p.nacc * (p.nt / 2 > 46 ? p.nt / 2 : 46);  // tensor pipe
@@ -439,6 +439,11 @@ static double swap_cost(int epi, int64_t N, int64_t K, const SwapPlan& p) {
   if (stage / feed > per_kb) per_kb = stage / feed;
   if (per_kb < 430.0) per_kb = 430.0;                              // issue
   if (epi == EPI_ROTARY) per_kb += 1.5 * p.nt;                     // measured: 16 k-blocks of 160 tokens 27 us, 64 of 176 52
+  return per_kb;
+}
+
+static double swap_cost(int epi, int64_t N, int64_t K, const SwapPlan& p) {
+  double per_kb = swap_per_kb(epi, p);
   if (p.stages <= 3) per_kb *= 1.2;                                // too shallow to hide a load
   const double chunks = p.nt / 16, warps = p.ew / 4;
   const double finish = 600.0 + chunks / warps * (epi == EPI_SILU_MUL ? 900.0 : epi == EPI_ROTARY ? 3000.0 : 350.0 * p.nacc);
@@ -459,6 +464,20 @@ static double swap_cost(int epi, int64_t N, int64_t K, const SwapPlan& p) {
   const double in_flight = (double)p.grid * p.stages * p.nacc * kSwapTileBytes / 3000.0;
   const double hbm = (double)N * K * 2 / (in_flight < 3500.0 ? in_flight : 3500.0) + 8000.0;
   return c > hbm ? c : hbm;
+}
+
+// Small batches are bound by the weights, and a round of tiles by its share of them or by the k-blocks of one tile: the last
+// round costs as much with one tile as with many.  (8 tokens x 19072 x 4096: 40 us, estimated 41; x 128256 x 4096: 164, 161;
+// SiLU, 8 x 38144 x 8192: 138, 137.)
+double swap_walk_clocks(int epi, int64_t K, const SwapPlan& p) {
+  const int64_t tiles = (int64_t)p.w_tiles * p.t_tiles, rounds = tiles / p.grid, left = tiles % p.grid;
+  const double chunks = p.nt / 16, warps = p.ew / 4, main = p.k_blocks * swap_per_kb(epi, p);
+  const double finish = epi == EPI_STORE ? 300.0 + chunks * 950.0 : 600.0 + chunks / warps * (epi == EPI_SILU_MUL ? 900.0 : 3000.0);
+  const double tile = main > finish ? main : finish, bytes = 2.0 * 128 * p.nacc * (double)K / p.t_tiles;
+  const double in_flight = (double)p.grid * p.stages * p.nacc * kSwapTileBytes / 3000.0, hbm = in_flight < 3500.0 ? in_flight : 3500.0;
+  double c = 6000.0 + finish + (double)rounds * (p.grid * bytes / hbm > tile ? p.grid * bytes / hbm : tile);
+  if (left) c += left * bytes / hbm > tile ? left * bytes / hbm : tile;
+  return c;
 }
 
 static bool swap_fits(int epi, int64_t M, int64_t N, int head_size, int neox) {

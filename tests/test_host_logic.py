@@ -602,7 +602,7 @@ def test_swapped_launches_are_consistent(T, epi, N, K):
     from sarathi_serve_b200 import dense_ops as D
     hd = 64 if N == 192 else 128
     p = D.gemm_launch(epi, T, N, K, hd)
-    assert p["kernel"] == "swapped" or T > 64
+    assert p["kernel"] == "swapped" or T > 64 or (epi == 0 and N > 148 * 128)  # (more tiles than SMs: an estimate decides)
     if p["kernel"] == "general":
         q = D.gemm_plan(epi, T, N, K, hd)
         assert {k: p[k] for k in q} == q
@@ -642,6 +642,9 @@ def test_which_kernel_a_projection_takes():
     for T, N, K in ((1185, 8, 64), (593, 9, 512), (1185, 8, 4160), (2369, 8, 4096), (65536, 1, 1024)):  # more rounds than pay off
         assert D.gemm_launch(0, T, N, K)["kernel"] != "narrow", (T, N, K)
     assert D.gemm_launch(0, 4, 17, 4096)["kernel"] == "swapped"
+    # 149 tiles: the second round of the swapped kernel has one; over 32 tokens its rings are too shallow to walk the vocabulary
+    assert D.gemm_launch(0, 8, 148 * 128, 4096)["kernel"] == "swapped" and D.gemm_launch(0, 8, 149 * 128, 4096)["kernel"] == "general"
+    assert D.gemm_launch(0, 8, 128256, 4096)["kernel"] == "swapped" and D.gemm_launch(0, 61, 128256, 4096)["kernel"] == "general"
     assert D.gemm_launch(0, 4, 8, 4100)["kernel"] == "swapped"                       # rows that are no multiple of 16 bytes
     assert D.gemm_launch(1, 4, 768, 4096, is_neox=False)["kernel"] == "general"      # pairs of a GPT-J head sit side by side
     assert D.gemm_launch(1, 300, 768, 4096, is_neox=False, tile_cfg=6064)["kernel"] == "general"
