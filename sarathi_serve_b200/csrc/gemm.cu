@@ -190,13 +190,13 @@ GemmPlan plan_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, int 
       int units_max = cta2 ? sms / 2 : sms;     // CTAs or CTA pairs that run at once
       if (cta2 && epi == EPI_PUSH && max_coresident_clusters(2) < units_max) units_max = max_coresident_clusters(2);
       const int64_t total = tiles * k_blocks;
-      // per-k-block clocks of one SM (constants fitted to the measured times of the full kernels on B200):
-      //   one CTA: about 616 clocks per k-block whatever N <= 256 -- not the tensor pipe (the MMA-rate probe of
-      //   diag.cu shows N/2 clocks per MMA for one CTA as for a pair) but the operand feed: a single-CTA stage
-      //   of 128 + N rows crosses L2 -> shared memory at ~50 B/clk/SM with every SM pulling;
+      // per-k-block clocks of one SM.  The constants date from when a k-block was issued under a lane test, which took about
+      // 550 clocks whatever the tile: hence 616 for one CTA.  Under an elected lane a CTA takes 2 * max(N, 92) clocks, or the
+      // feed of its stage (gemm_plan_clocks).  They are not refitted: they only rank this kernel's own plans, and what is
+      // set against the swapped kernel is gemm_plan_clocks of the plan chosen here.
       //   a CTA pair loads half of the B tile per SM and reaches the nominal N/2 clocks per MMA down to a
-      //   floor of ~65; its 256x256 tiles are again bound by the feed (64 B/clk needed), and shared memory
-      //   itself (fill + operand reads) is modelled too.
+      //   floor of ~65; its 256x256 tiles are bound by the feed (64 B/clk needed, ~50 with every SM pulling), and shared
+      //   memory itself (fill + operand reads) is modelled too.
       const double stage = gemm_stage_bytes(mi, bn, cta2);
       const double mma_nominal = cta2 ? 2.0 * mi * bn : 616.0 * mi;
       const double mma_floor = cta2 ? 260.0 * mi : 616.0 * mi;
@@ -207,7 +207,7 @@ GemmPlan plan_gemm(int epi, int64_t M, int64_t N, int64_t K, int head_size, int 
       if (stage / 50.0 > per_kb) per_kb = stage / 50.0;
       const int64_t busy_sms = (tiles < units_max ? tiles : units_max) * (cta2 ? 2 : 1);
       if (busy_sms > sms / 2) per_kb *= 1.0 + 0.25 * (double)(busy_sms - sms / 2) / (sms / 2);  // L2 contention
-      if (mi == 2) per_kb *= 1.4;  // single-buffered accumulators, shallow ring: measured well above the model
+      if (mi == 2) per_kb *= 1.4;  // single-buffered accumulators, shallow ring: measured (then) well above the model
       const double epi_units = (mi == 2 ? bn / 32.0 : bn / 64.0);
       const double epi_c = epi_units * 450.0 + 400.0;
       const bool dbuf = mi * bn * 2 <= 512;
